@@ -382,7 +382,7 @@ frontend_kernel(FrontArgs a) {
       float *dst = a.out + (cd.frame_off + t) * (long long)a.n_mels;
       const float ref_db = 10.0f * log10f(a.ref);
       if (walk) {
-        // the warp kernel's filterbank walk (tables at build_mel_lane_kernel):
+        // the filterbank walk (tables at build_mel_lane_kernel):
         // thread j < TW sums its 32 bins into part slots, segment heads take
         // the parts of the threads they run into, a band is two slot reads
         float2 *parts = reinterpret_cast<float2 *>(P + 33 * TW);
@@ -921,7 +921,7 @@ __global__ void build_mel_seg_kernel(int2 *seg, const int *bin_seg, const int4 *
   ok[1] = good;
 }
 
-// Lane tables of the warp kernel's filterbank walk (one thread).  Lane l of a
+// Lane tables of the filterbank walk (one thread).  Lane l of a
 // frame group owns bins [32 l, 32 l + 32) (the last lane also the Nyquist bin
 // M = 32 tpf); it accumulates (R, F) = sum of (w2.x P, w2.y P) and stores the
 // pair in the next "part" slot wherever the segment of bin k differs from that

@@ -49,14 +49,14 @@ struct DevTables {
   float *mel_pw = nullptr;     // packed nonzero weights, row after row
   int4 *mel_info = nullptr;    // per mel {start bin, count, packed offset, nan-row flag}
   int mel_nnz = 0;             // entries of mel_pw
-  // Per-bin split of the same filterbank (warp kernel): bin k feeds band s(k)
+  // Per-bin split of the same filterbank (lane walk): bin k feeds band s(k)
   // with mel_w2[k].x and band s(k)-1 with mel_w2[k].y.  Segment s = the bins
   // [mel_seg[s].x, mel_seg[s+1].x) (n_mels + 1 entries; .y = NaN-row flag of
   // band s).
   float2 *mel_w2 = nullptr;
   int2 *mel_seg = nullptr;
   int mel_seg_ok = 0;          // 0: the split does not describe the filterbank (use mel_pw)
-  // Lane tables of the same split for the warp kernel (n_fft 256..2048): lane
+  // Lane tables of the same split for the filterbank walk (n_fft 256..4096): lane
   // l of a frame owns bins [32 l, 32 l + 32) and sums them into per-segment
   // parts (layout at build_mel_lane_kernel).
   float2 *mel_lw = nullptr;    // [33][n_fft/64] weights, lane-minor
@@ -100,6 +100,7 @@ struct FrontArgs {
   // DFT_GEMM_F16X3 only: per frame (frame-major, as the log-mel rows) the
   // power of two the frame's samples are scaled by before the fp16 split
   float *frame_scale = nullptr;
+  int even_starts = 0;  // 1: every clip's sig_off is even
   // error word of kernels with bounded waits (tensor-core frame kernel)
   unsigned *err = nullptr;
 };
@@ -152,26 +153,25 @@ cudaError_t launch_stack_memory(const float *x, float *y, int n_features, int n_
 int frames_per_tile(int log2n, int variant);
 // Number of launch variants the autotuner may choose from (1 = not tunable).
 int frame_variants(int log2n, int mode, int power_is_2);
-// Launch variant 3: the warp-per-frame kernel (MODE_MELDB, n_fft 256..2048).
+// Launch variant 3 (MODE_MELDB): the frame-pair kernel for n_fft 256..2048, the
+// warp-pair kernel for 4096.
 constexpr int kWarpVariant = 3;
 // Launch variant of the tensor-core frame kernel (n_fft 2048, MFCC path):
 // both 32-point DFT stages as fp16x3 tcgen05 GEMMs, 16 frames per tile.
 constexpr int kTcVariant = 5;
 constexpr int kTcFramesPerTile = 16;
-int warp_frames_per_tile(int log2n);  // 0 when the size has no warp kernel
+int warp_frames_per_tile(int log2n);  // variant 3; 0 when the size has none
 // Walking lanes of the filterbank walk (n_fft / 64, 32 bins each) for n_fft
-// 256..4096, else 0: the warp kernel's lanes (up to 2048), or the first
-// n_fft / 64 threads of a frame in the CTA-tile kernel.
+// 256..4096, else 0: the lanes of a frame pair (up to 2048) or of a warp pair,
+// or the first n_fft / 64 threads of a frame in the CTA-tile kernel.
 inline int mel_lane_tpf(int n_fft) {
   return (n_fft >= 256 && n_fft <= 4096 && (n_fft & (n_fft - 1)) == 0) ? n_fft / 64 : 0;
 }
-// Filterbank part slots that fit behind the padded spectrum (ps tpf floats,
-// ps = 36 for tpf = 32 and 33 below): in a warp-kernel frame buffer (at
-// least 66 tpf floats, frame group g starting tpf g floats in) for tpf <= 32
-// (480 at tpf 32, also within the CTA-tile and tensor-core kernels' larger
-// buffers); 1024
-// (the slot field's range) for tpf = 64, whose CTA-tile frame buffer holds
-// more than 33 tpf + 2048 floats.
+// Filterbank part slots that fit behind the padded spectrum in every kernel
+// that walks: 480 at tpf 32 (the frame-pair kernel's 1 024 16-byte slots less
+// the spectrum's 17 tpf; the CTA-tile and tensor-core kernels hold more), 17
+// tpf - 16 below, 1 024 (the slot field's range) at tpf 64, whose CTA-tile
+// frame buffer holds more than 33 tpf + 2048 floats.
 inline int mel_lane_max_slots(int tpf) {
   if (tpf <= 0) return 0;
   if (tpf > 32) return 1024;
@@ -179,6 +179,8 @@ inline int mel_lane_max_slots(int tpf) {
   return (66 * tpf - ps * tpf - tpf * (32 / tpf - 1)) / 2;
 }
 cudaError_t launch_frontend_tc(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched);
+cudaError_t launch_frontend_pair(int log2n, const FrontArgs &a, int grid_limit, cudaStream_t s,
+                                 int *launched);
 cudaError_t launch_frontend_warp(int log2n, const FrontArgs &a, int grid_limit, cudaStream_t s,
                                  int *launched);
 // Stockham twiddle table length (entries) for log2(n_fft) >= 5.

@@ -234,6 +234,7 @@ extern "C" MM_API int32_t mm_mfcc_noalloc(const float *d_signal, int64_t signal_
   a.ref = g.ref;
   a.out = meldb;
   a.clip_max = clip_max;
+  a.even_starts = sig_off == 0;
   if ((e = launch_frontend(g.log2n, MODE_MELDB, g.variant, a, 0, s, nullptr)) != cudaSuccess)
     return cuda_status(e);
 

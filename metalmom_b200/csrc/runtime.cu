@@ -318,6 +318,7 @@ cudaError_t enqueue_batch(const Group &g, const Layout &L, const DevTables *t, c
   a.out = (g.mode == MODE_MELDB) ? b.meldb : b.out;
   a.clip_max = b.clip_max;
   a.err = t->dft_err;
+  a.even_starts = 1;  // make_layout puts every clip at a multiple of 4 samples
   int grid = 0;
   if (g.dft_form == DFT_GEMM_F16X3 && g.mode == MODE_MELDB) {
     a.frame_scale = b.frame_scale;
