@@ -34,23 +34,27 @@ int gpu_available() {
 }
 
 namespace {
-// Untuned launch variant per log2(n_fft): the warp kernels (variant 3) for
-// n_fft 2048 and 4096, the fastest there on B200 and within the reference's
-// elementwise MFCC goldens by a wide margin; variant 0 elsewhere.  At n_fft
-// 1024 the warp kernel's float32 FFT noise puts one small coefficient of the
-// 440 Hz golden (13 MFCC, 40 bands) just past its 1e-4 bound, where the
-// CTA-tile kernel stays inside it; the autotuner may still pick it.  A mode
-// without variant 3 falls back to 0.
+// What mm_tune_set or mm_autotune last stored per log2(n_fft), as mm_tune_get
+// reports it, and whether either has run for that size.
 std::atomic<int> g_tuned[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, kWarpVariant, kWarpVariant, 0, 0, 0};
+std::atomic<bool> g_tuned_set[16];
 }
 
 int tuned_variant(int log2n) { return (log2n >= 0 && log2n < 16) ? g_tuned[log2n].load() : 0; }
 void set_tuned_variant(int log2n, int v) {
-  if (log2n >= 0 && log2n < 16) g_tuned[log2n].store(v);
+  if (log2n < 0 || log2n >= 16) return;
+  g_tuned[log2n].store(v);
+  g_tuned_set[log2n].store(true);
 }
 int group_variant(const Group &g) {
   if (g.dft_form != DFT_FFT_F32) return kDftVariant;
   const int nv = frame_variants(g.log2n, g.mode, g.power == 2.0f);
+  // Untuned: variant 3 wherever it exists (MFCC path, n_fft 256..4096).  Whole
+  // step against variant 0 on 64 clips of 30 s (hop n_fft/4): n_fft 256 323 /
+  // 520 us, 512 253 / 410, 1024 225 / 441, 2048 218 / 428, 4096 289 / 449; on
+  // one clip of 1 to 30 s between equal and 1.5x faster (n_fft 256 and 512 with
+  // few frames: within one 2 us step either way).
+  if (g.log2n < 16 && !g_tuned_set[g.log2n].load()) return nv > kWarpVariant ? kWarpVariant : 0;
   const int v = tuned_variant(g.log2n);
   if (v == kTcVariant)  // the tensor-core kernel: n_fft 2048 on the MFCC path only
     return (g.log2n == 11 && g.mode == MODE_MELDB && g.power == 2.0f) ? kTcVariant : (nv > kWarpVariant ? kWarpVariant : 0);
