@@ -230,17 +230,17 @@ static int32_t db_common(const float *data, int64_t count, float mult, float ref
   const size_t bytes = sizeof(float) * (size_t)count;
   const size_t seg = ((bytes + 255) / 256) * 256;
   Workspace *ws = nullptr;
-  if ((st = thread_workspace(2 * seg + 256, bytes, &ws)) != MM_OK) return st;
+  const size_t scratch = db_scratch_bytes(count, amin, false, top_db);
+  if ((st = thread_workspace(2 * seg + scratch + 256, bytes, &ws)) != MM_OK) return st;
   cudaStream_t s = ws->stream;
   cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e);
   float *d_x = reinterpret_cast<float *>(ws->dev);
   float *d_y = reinterpret_cast<float *>(ws->dev + seg);
-  unsigned *slot = reinterpret_cast<unsigned *>(ws->dev + 2 * seg);
   memcpy(ws->host, data, bytes);
   if ((e = cudaMemcpyAsync(d_x, ws->host, bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
     return cuda_status(e);
-  if ((e = launch_db(d_x, d_y, count, mult, amin, ref, top_db, slot, s)) != cudaSuccess)
+  if ((e = launch_db(d_x, d_y, count, mult, amin, ref, false, top_db, ws->dev + 2 * seg, s)) != cudaSuccess)
     return cuda_status(e);
   if ((e = cudaMemcpyAsync(ws->host, d_y, bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return cuda_status(e);

@@ -220,12 +220,13 @@ cudaError_t launch_fill_u32(unsigned *p, unsigned v, long long n, cudaStream_t s
 // Deterministic pseudo-random samples in [-0.5, 0.5) (autotuning inputs).
 cudaError_t launch_fill_pattern(float *p, long long n, cudaStream_t s);
 
-// dB scaling over a flat array: pass 1 writes mult*log10(max(x,amin)/ref) and the
-// encoded max into *slot; pass 2 floors at max - top_db.
-// ref_slot (2 words, optional): take the reference value as max(x) on the device.
-cudaError_t launch_db(const float *x, float *y, long long n, float mult, float amin,
-                      float ref, float top_db, unsigned *slot, cudaStream_t s,
-                      unsigned *ref_slot = nullptr);
+// dB scaling over a flat array: y = mult*log10(max(x,amin)/ref), floored at
+// max(y) - top_db when top_db > 0; ref_max: ref is max(x), taken on the device
+// (NaN when x holds one).  y may be x.  scratch: db_scratch_bytes (same
+// arguments) bytes, 8-byte aligned; may be null when that is 0.
+size_t db_scratch_bytes(long long n, float amin, bool ref_max, float top_db);
+cudaError_t launch_db(const float *x, float *y, long long n, float mult, float amin, float ref, bool ref_max,
+                      float top_db, void *scratch, cudaStream_t s);
 cudaError_t build_mel_dense(float *W, int4 *info, int sr, int n_fft, int n_mels, float fmin, float fmax,
                             cudaStream_t s);
 cudaError_t build_dct_basis_rows(float *B, int n_out, int n_rows, cudaStream_t s);
