@@ -111,30 +111,35 @@ int warp_frames_per_tile(int log2n) {
 
 // Samples (x[i], x[i+1]) for i = first + stride r, r < Q, with the padding
 // rule; used only for frames that overlap the clip's edges.  Out of line, so
-// that its index arithmetic does not weigh on the interior path, and unrolled,
-// so that its loads are in flight together (a short clip waits for its edges).
+// that its index arithmetic does not weigh on the interior path, and fully
+// unrolled, so that its loads are in flight together (a short clip waits for
+// its edges).
 template <int Q>
 __device__ __noinline__ void gather_edge_n(float2 *out, const float *sig, long long first, long long L, int pad_mode,
                                            int stride) {
   const long long last = first + (long long)stride * (Q - 1) + 1;
-  const bool reflect = pad_mode == PAD_REFLECT;
-  if (reflect && (first <= -L || last > 2 * (L - 1))) {  // more than one reflection: a clip shorter than the padding
+  // the clip as offsets [lo, hi) from `first` (the offsets asked for are small)
+  constexpr long long kFar = 1 << 30;
+  const int lo = (int)max(min(-first, kFar), -kFar), hi = (int)max(min(L - first, kFar), -kFar);
+  const float *p = sig + first;
+  if (pad_mode != PAD_REFLECT) {
+#pragma unroll
+    for (int r = 0; r < Q; r++) {
+      const int i = stride * r;
+      float x = 0.0f, y = 0.0f;
+      if (i >= lo && i < hi) x = __ldg(p + i);
+      if (i + 1 >= lo && i + 1 < hi) y = __ldg(p + i + 1);
+      out[r] = make_float2(x, y);
+    }
+  } else if (first > -L && last <= 2 * (L - 1)) {  // one reflection at most
+    auto at = [&](int i) { return i < lo ? 2 * lo - i : (i >= hi ? 2 * (hi - 1) - i : i); };
+#pragma unroll
+    for (int r = 0; r < Q; r++) out[r] = make_float2(__ldg(p + at(stride * r)), __ldg(p + at(stride * r + 1)));
+  } else {  // a clip shorter than the padding
     for (int r = 0; r < Q; r++) {
       const long long n0 = first + (long long)stride * r;
       out[r] = make_float2(sample_at(sig, n0, L, pad_mode), sample_at(sig, n0 + 1, L, pad_mode));
     }
-    return;
-  }
-  auto at = [&](long long i) {  // index inside the clip, -1 in zero padding
-    if (i >= 0 && i < L) return i;
-    return reflect ? (i < 0 ? -i : 2 * (L - 1) - i) : -1LL;
-  };
-#pragma unroll 8
-  for (int r = 0; r < Q; r++) {
-    const long long n0 = first + (long long)stride * r;
-    const long long i0 = at(n0), i1 = at(n0 + 1);
-    const float x = __ldg(sig + (i0 >= 0 ? i0 : 0)), y = __ldg(sig + (i1 >= 0 ? i1 : 0));
-    out[r] = make_float2(i0 >= 0 ? x : 0.0f, i1 >= 0 ? y : 0.0f);
   }
 }
 
