@@ -3,6 +3,7 @@
 // Every wait is bounded: a wait that runs out returns false and the caller
 // records an error instead of spinning on.
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace mm {
@@ -70,6 +71,34 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Programmatic dependent launch.  A kernel launched with launch_after may
+// start while the kernel before it in the stream finishes; griddep_wait
+// returns once that kernel has completed and its writes are visible (at once
+// when there is nothing to wait for).  griddep_launch lets the next such kernel
+// start early.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launch `kern` (see above: 3 s of music, host call to host result, 72.8 -> 68.3 us
+// with both the frame kernel and the DCT launched this way; a graph replay of
+// 64 clips of 30 s 226 -> 223 us), which calls griddep_wait before it reads or writes anything
+// that an earlier kernel touches.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s,
+                                A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 }  // namespace mm

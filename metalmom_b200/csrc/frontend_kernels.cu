@@ -1381,6 +1381,7 @@ __global__ void __launch_bounds__(256, 2) dct_pipe_kernel(DctArgs a) {
   }
   const float4 *brow = reinterpret_cast<const float4 *>(bas + kg * KQ * nm);
   const float4 *trow = reinterpret_cast<const float4 *>(tile + fr * stride);
+  griddep_wait();  // the basis is constant; the log-mel rows and maxima come from the frame kernel
   int ti = blockIdx.x;
   if (ti >= a.total_tiles) return;
   float4 pre[kDctPipeVec];
@@ -1500,6 +1501,7 @@ __global__ void __launch_bounds__(128, S == 2 ? 3 : 2) dct_fold2_kernel(DctArgs 
     const int k = coef(row / KQ, row % KQ);
     bas[i] = k < a.n_mfcc ? __ldg(a.basis + (long long)k * NM + n) : 0.0f;
   }
+  griddep_wait();  // the basis is constant; the log-mel rows and maxima come from the frame kernel
   int ti = blockIdx.x;
   if (ti >= a.total_tiles) return;
   // A tile's meta takes three dependent loads (tile -> clip -> descriptor and
@@ -1631,8 +1633,7 @@ static cudaError_t launch_dct_fold2_s(const DctArgs &a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   long long grid = (long long)sms * per_sm;
   if (grid > a.total_tiles) grid = a.total_tiles;
-  dct_fold2_kernel<KQ, S, NM><<<(unsigned)grid, 128, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(dct_fold2_kernel<KQ, S, NM>, (unsigned)grid, 128, smem, s, a);
 }
 
 // n_mels 64, 80 or 128 (the bands of the default, speech and mixed-batch front ends)
@@ -1654,8 +1655,7 @@ static cudaError_t launch_dct_pipe_t(const DctArgs &a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   long long grid = (long long)sms * per_sm;
   if (grid > a.total_tiles) grid = a.total_tiles;
-  kern<<<(unsigned)grid, 256, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(kern, (unsigned)grid, 256, smem, s, a);
 }
 
 template <int KQ>

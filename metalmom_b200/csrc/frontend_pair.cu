@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
   using S = PShape<LOG2N>;
   constexpr int N = S::N, M = S::M, TPF = S::TPF, C = S::C, HALF = S::HALF, PS = S::PS;
   constexpr unsigned FULL = 0xffffffffu;
+  griddep_launch();
   extern __shared__ __align__(16) unsigned char smem[];
   const int nmel = a.n_mels;
   const float ref_db = 10.0f * log10f(a.ref);
@@ -269,6 +270,7 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
   const int *band = staged ? words_s : src_words;
   const float *melw = reinterpret_cast<const float *>(band);
   twice = __syncthreads_or(twice) != 0;
+  griddep_wait();  // the tables are constant; the clips and their maxima are not
   if (warp >= nw) return;  // a small batch: this warp only helped to stage the tables
 
   // real-split bases W_N^(first bin of each column pair), C > 1
@@ -679,7 +681,8 @@ static cudaError_t launch_pair_d(const FrontArgs &a, int grid_limit, cudaStream_
   if (grid_limit > 0 && grid > grid_limit) grid = grid_limit;
   if (grid > units) grid = units;
   if (grid < 1) return cudaSuccess;
-  kern<<<(unsigned)grid, 32 * S::NW, smem, s>>>(a, nw);
+  e = launch_after(kern, (unsigned)grid, 32 * S::NW, smem, s, a, nw);
+  if (e != cudaSuccess) return e;
   if (launched) *launched = (int)grid;
   return cudaGetLastError();
 }
