@@ -62,6 +62,12 @@ typedef void* mm_context;
 /* Replaces MetalMomBridge/Bridge.swift:22 (mm_init). */
 MM_API mm_context mm_init(void);
 
+/* Additive: as mm_init, but large results of calls on this context may lie in
+ * page-locked blocks that the library keeps and reuses (64 MB at most; past
+ * that they are malloc'd as usual), so that they arrive without a host copy.
+ * Release them with mm_buffer_free and nothing else. */
+MM_API mm_context mm_init_pooled(void);
+
 /* Replaces Bridge.swift:33 (mm_destroy); destroying twice is a no-op. */
 MM_API void mm_destroy(mm_context ctx);
 

@@ -9,7 +9,7 @@
 
 #include <algorithm>
 #include <mutex>
-#include <unordered_set>
+#include <unordered_map>
 #include <vector>
 
 #include "runtime.h"
@@ -23,11 +23,19 @@ struct Context {
   int magic = 0x4d4d4232;
 };
 std::mutex g_ctx_mu;
-std::unordered_set<void *> g_ctx;
+std::unordered_map<const void *, bool> g_ctx;  // context -> its results may be pooled
+
+mm_context new_context(bool pooled) {
+  Context *c = new (std::nothrow) Context();
+  if (!c) return nullptr;
+  std::lock_guard<std::mutex> lock(g_ctx_mu);
+  g_ctx[c] = pooled;
+  return c;
+}
 
 // Run one clip (n = 1) or a batch of clips through `g`; on success *outs[i]
 // holds a malloc'd [rows x n_frames_i] block (NULL when empty).
-int run_batch(const Group &g_in, const float *const *signals, const int64_t *lengths, int n,
+int run_batch(mm_context ctx, const Group &g_in, const float *const *signals, const int64_t *lengths, int n,
               float **outs) {
   for (int i = 0; i < n; i++) outs[i] = nullptr;
   Group g = g_in;
@@ -44,7 +52,7 @@ int run_batch(const Group &g_in, const float *const *signals, const int64_t *len
   const size_t desc_bytes = carve_arena(g, L, nullptr, probe);
   const size_t sig_bytes = sizeof(float) * (size_t)L.sig_elems;
   const size_t out_bytes = sizeof(float) * (size_t)L.out_elems;
-  const size_t host_bytes = std::max(sig_bytes + desc_bytes, out_bytes) + 256;
+  const size_t host_bytes = std::max(sig_bytes + desc_bytes, n > 1 ? out_bytes : 0) + 256;
   Workspace *ws = nullptr;
   if ((st = thread_workspace(dev_bytes, host_bytes, &ws)) != MM_OK) return st;
   DevBatch b;
@@ -60,7 +68,7 @@ int run_batch(const Group &g_in, const float *const *signals, const int64_t *len
   // The staged region (which spans the large clips' slots too) is uploaded
   // first, so that the direct copies, later in stream order, land on top.
   char *h = ws->host;
-  constexpr size_t kDirect = size_t(1) << 20;
+  constexpr size_t kDirect = kDirectUpload;
   bool staged = false;
   for (int i = 0; i < n; i++) {
     const size_t bytes = sizeof(float) * (size_t)lengths[i];
@@ -82,6 +90,14 @@ int run_batch(const Group &g_in, const float *const *signals, const int64_t *len
   if ((e = cudaMemcpyAsync(b.clips, h + sig_bytes, desc_bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
     return cuda_status(e);
   if ((e = enqueue_batch(g, L, t, b, s, nullptr, nullptr)) != cudaSuccess) return cuda_status(e);
+  if (n == 1) {
+    if ((st = fetch_result(b.out, out_bytes, context_pooled(ctx), ws, &outs[0])) != MM_OK) return st;
+    if ((st = take_error_word(g, t)) != MM_OK) {
+      result_free(outs[0]);
+      outs[0] = nullptr;
+    }
+    return st;
+  }
   if ((e = cudaMemcpyAsync(h, b.out, out_bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
     return cuda_status(e);
   if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_status(e);
@@ -123,15 +139,17 @@ bool supported_size(const Group &g) { return g.log2n <= 15; }
 
 }  // namespace
 
+bool mm::context_pooled(const void *ctx) {
+  std::lock_guard<std::mutex> lock(g_ctx_mu);
+  auto it = g_ctx.find(ctx);
+  return it != g_ctx.end() && it->second;
+}
+
 extern "C" {
 
-mm_context mm_init(void) {
-  Context *c = new (std::nothrow) Context();
-  if (!c) return nullptr;
-  std::lock_guard<std::mutex> lock(g_ctx_mu);
-  g_ctx.insert(c);
-  return c;
-}
+mm_context mm_init(void) { return new_context(false); }
+
+mm_context mm_init_pooled(void) { return new_context(true); }
 
 void mm_destroy(mm_context ctx) {
   if (!ctx) return;
@@ -144,7 +162,7 @@ void mm_destroy(mm_context ctx) {
 
 void mm_buffer_free(MMBuffer *buf) {
   if (!buf) return;
-  free(buf->data);
+  result_free(buf->data);
   buf->data = nullptr;
   buf->ndim = 0;
   buf->dtype = 0;
@@ -174,7 +192,7 @@ int32_t mm_stft(mm_context ctx, const float *signal_data, int64_t signal_length,
   const long long rows = n_fft / 2 + 1;
   float *data = nullptr;
   if (T > 0) {
-    int st = run_batch(g, &signal_data, &signal_length, 1, &data);
+    int st = run_batch(ctx, g, &signal_data, &signal_length, 1, &data);
     if (st != MM_OK) return st;
   }
   fill_buffer(out, data, rows, T);
@@ -212,7 +230,7 @@ int32_t mm_stft_complex(mm_context ctx, const float *signal_data, int64_t signal
   if (T > 0 && !supported_size(g)) return MM_ERR_INVALID_INPUT;
   float *data = nullptr;
   if (T > 0) {
-    int st = run_batch(g, &signal_data, &signal_length, 1, &data);
+    int st = run_batch(ctx, g, &signal_data, &signal_length, 1, &data);
     if (st != MM_OK) return st;
   }
   fill_buffer(out, data, nfreq, T);
@@ -222,7 +240,7 @@ int32_t mm_stft_complex(mm_context ctx, const float *signal_data, int64_t signal
   return MM_OK;
 }
 
-static int32_t db_common(const float *data, int64_t count, float mult, float ref, float amin,
+static int32_t db_common(mm_context ctx, const float *data, int64_t count, float mult, float ref, float amin,
                          float top_db, MMBuffer *out) {
   if (!data || count <= 0 || !out) return MM_ERR_INVALID_INPUT;
   int st = gpu_available();
@@ -231,23 +249,17 @@ static int32_t db_common(const float *data, int64_t count, float mult, float ref
   const size_t seg = ((bytes + 255) / 256) * 256;
   Workspace *ws = nullptr;
   const size_t scratch = db_scratch_bytes(count, amin, false, top_db);
-  if ((st = thread_workspace(2 * seg + scratch + 256, bytes, &ws)) != MM_OK) return st;
+  if ((st = thread_workspace(2 * seg + scratch + 256, upload_staging(bytes), &ws)) != MM_OK) return st;
   cudaStream_t s = ws->stream;
   cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e);
   float *d_x = reinterpret_cast<float *>(ws->dev);
   float *d_y = reinterpret_cast<float *>(ws->dev + seg);
-  memcpy(ws->host, data, bytes);
-  if ((e = cudaMemcpyAsync(d_x, ws->host, bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
-    return cuda_status(e);
+  if ((e = upload(d_x, data, bytes, ws)) != cudaSuccess) return cuda_status(e);
   if ((e = launch_db(d_x, d_y, count, mult, amin, ref, false, top_db, ws->dev + 2 * seg, s)) != cudaSuccess)
     return cuda_status(e);
-  if ((e = cudaMemcpyAsync(ws->host, d_y, bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-    return cuda_status(e);
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_status(e);
-  float *res = (float *)malloc(bytes);
-  if (!res) return MM_ERR_ALLOC_FAILED;
-  memcpy(res, ws->host, bytes);
+  float *res = nullptr;
+  if ((st = fetch_result(d_y, bytes, context_pooled(ctx), ws, &res)) != MM_OK) return st;
   fill_buffer(out, res, count, 0);
   out->ndim = 1;
   out->shape[1] = 0;
@@ -257,14 +269,13 @@ static int32_t db_common(const float *data, int64_t count, float mult, float ref
 
 int32_t mm_power_to_db(mm_context ctx, const float *data, int64_t count, float ref, float amin,
                        float top_db, MMBuffer *out) {
-  (void)ctx;  // the reference does not check the context here (Bridge.swift:276-278)
-  return db_common(data, count, 10.0f, ref, amin, top_db, out);
+  // the reference does not check the context here (Bridge.swift:276-278)
+  return db_common(ctx, data, count, 10.0f, ref, amin, top_db, out);
 }
 
 int32_t mm_amplitude_to_db(mm_context ctx, const float *data, int64_t count, float ref, float amin,
                            float top_db, MMBuffer *out) {
-  (void)ctx;
-  return db_common(data, count, 20.0f, ref, amin, top_db, out);
+  return db_common(ctx, data, count, 20.0f, ref, amin, top_db, out);
 }
 
 int32_t mm_mel_spectrogram(mm_context ctx, const float *signal_data, int64_t signal_length,
@@ -282,7 +293,7 @@ int32_t mm_mel_spectrogram(mm_context ctx, const float *signal_data, int64_t sig
   float *data = nullptr;
   if (T > 0 && n_mels > 0) {
     if (!supported_size(g)) return MM_ERR_INVALID_INPUT;
-    st = run_batch(g, &signal_data, &signal_length, 1, &data);
+    st = run_batch(ctx, g, &signal_data, &signal_length, 1, &data);
     if (st != MM_OK) return st;
   }
   fill_buffer(out, data, n_mels, T);
@@ -307,7 +318,7 @@ int32_t mm_mfcc(mm_context ctx, const float *signal_data, int64_t signal_length,
   float *data = nullptr;
   if (T > 0 && g.n_mfcc_eff > 0) {
     if (!supported_size(g)) return MM_ERR_INVALID_INPUT;
-    st = run_batch(g, &signal_data, &signal_length, 1, &data);
+    st = run_batch(ctx, g, &signal_data, &signal_length, 1, &data);
     if (st != MM_OK) return st;
   }
   fill_buffer(out, data, g.n_mfcc_eff, T);
@@ -361,28 +372,22 @@ static bool savgol_coeffs(int width, int order, float *out) {
 
 // Host matrix in -> kernel -> host matrix out through the thread's workspace.
 template <typename Launch>
-static int32_t run_matrix(const float *data, size_t in_count, size_t out_count, long long rows, long long cols,
+static int32_t run_matrix(mm_context ctx, const float *data, size_t in_count, size_t out_count, long long rows, long long cols,
                           MMBuffer *out, Launch launch) {
   int st = gpu_available();
   if (st != MM_OK) return st;
   const size_t in_b = sizeof(float) * in_count, out_b = sizeof(float) * out_count;
   const size_t in_pad = (in_b + 255) & ~size_t(255);
   Workspace *ws = nullptr;
-  if ((st = thread_workspace(in_pad + out_b, std::max(in_b, out_b), &ws)) != MM_OK) return st;
+  if ((st = thread_workspace(in_pad + out_b, upload_staging(in_b), &ws)) != MM_OK) return st;
   cudaStream_t s = ws->stream;
   cudaError_t e = cudaStreamSynchronize(s);
   float *d_in = reinterpret_cast<float *>(ws->dev), *d_out = reinterpret_cast<float *>(ws->dev + in_pad);
-  if (e == cudaSuccess) {
-    memcpy(ws->host, data, in_b);
-    e = cudaMemcpyAsync(d_in, ws->host, in_b, cudaMemcpyHostToDevice, s);
-  }
+  if (e == cudaSuccess) e = upload(d_in, data, in_b, ws);
   if (e == cudaSuccess) e = launch(d_in, d_out, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(ws->host, d_out, out_b, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e);
-  float *res = (float *)malloc(out_b);
-  if (!res) return MM_ERR_ALLOC_FAILED;
-  memcpy(res, ws->host, out_b);
+  float *res = nullptr;
+  if ((st = fetch_result(d_out, out_b, context_pooled(ctx), ws, &res)) != MM_OK) return st;
   fill_buffer(out, res, rows, cols);
   return MM_OK;
 }
@@ -400,7 +405,7 @@ extern "C" {
 int32_t mm_onset_strength(mm_context ctx, const float *signal_data, int64_t signal_length, int32_t sample_rate,
                           int32_t n_fft, int32_t hop_length, int32_t n_mels, float f_min, float f_max,
                           int32_t center, int32_t aggregate, MMBuffer *out) {
-  (void)ctx;  // the reference ignores the context here too
+  // (the reference ignores the context here too)
   if (!signal_data || signal_length <= 0 || !out) return MM_ERR_INVALID_INPUT;
   if (n_mels <= 0) return MM_ERR_INVALID_INPUT;  // the reference would average over no bands
   Group g;
@@ -420,7 +425,7 @@ int32_t mm_onset_strength(mm_context ctx, const float *signal_data, int64_t sign
   float *data = nullptr;
   if (T > 0) {
     if (!supported_size(g)) return MM_ERR_INVALID_INPUT;
-    st = run_batch(g, &signal_data, &signal_length, 1, &data);
+    st = run_batch(ctx, g, &signal_data, &signal_length, 1, &data);
     if (st != MM_OK) return st;
     fill_buffer(out, data, rows, T);
     return MM_OK;
@@ -437,14 +442,13 @@ int32_t mm_onset_strength(mm_context ctx, const float *signal_data, int64_t sign
 // n_frames < width.
 int32_t mm_delta(mm_context ctx, const float *data, int64_t count, int32_t n_features, int32_t n_frames,
                  int32_t width, int32_t order, MMBuffer *out) {
-  (void)ctx;
   if (!data || count <= 0 || !out || n_features <= 0 || n_frames <= 0) return MM_ERR_INVALID_INPUT;
   if ((long long)n_features * n_frames != count) return MM_ERR_INVALID_INPUT;
   if (width < 3 || width % 2 == 0 || width > kDeltaMaxWidth || order < 1 || order >= width || n_frames < width)
     return MM_ERR_INVALID_INPUT;
   DeltaCoeffs c{};
   if (!savgol_coeffs(width, order, c.c)) return MM_ERR_INVALID_INPUT;
-  return run_matrix(data, (size_t)count, (size_t)count, n_features, n_frames, out,
+  return run_matrix(ctx, data, (size_t)count, (size_t)count, n_features, n_frames, out,
                     [&](const float *x, float *y, cudaStream_t s) {
                       return launch_delta(x, y, n_features, n_frames, width, c, s);
                     });
@@ -454,11 +458,10 @@ int32_t mm_delta(mm_context ctx, const float *data, int64_t count, int32_t n_fea
 // n_frames], zeros before the start.
 int32_t mm_stack_memory(mm_context ctx, const float *data, int64_t count, int32_t n_features, int32_t n_frames,
                         int32_t n_steps, int32_t delay, MMBuffer *out) {
-  (void)ctx;
   if (!data || count <= 0 || !out || n_features <= 0 || n_frames <= 0 || n_steps <= 0) return MM_ERR_INVALID_INPUT;
   if ((long long)n_features * n_frames != count) return MM_ERR_INVALID_INPUT;
   const size_t out_count = (size_t)count * (size_t)n_steps;
-  return run_matrix(data, (size_t)count, out_count, (long long)n_features * n_steps, n_frames, out,
+  return run_matrix(ctx, data, (size_t)count, out_count, (long long)n_features * n_steps, n_frames, out,
                     [&](const float *x, float *y, cudaStream_t s) {
                       return launch_stack_memory(x, y, n_features, n_frames, n_steps, delay, s);
                     });
@@ -502,7 +505,7 @@ int32_t mm_mfcc_batch(mm_context ctx, const float *const *signals, const int64_t
   if (st != MM_OK) return st;
   std::vector<float *> data(n_clips, nullptr);
   if (g.n_mfcc_eff > 0) {
-    st = run_batch(g, signals, lengths, n_clips, data.data());
+    st = run_batch(ctx, g, signals, lengths, n_clips, data.data());
     if (st != MM_OK) return st;
   }
   for (int i = 0; i < n_clips; i++)

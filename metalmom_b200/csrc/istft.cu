@@ -149,24 +149,17 @@ int32_t mm_istft(mm_context ctx, const float *stft_data, int64_t stft_count, int
     out->count = 0;
     return MM_OK;
   }
-  float *res = (float *)calloc((size_t)out_len, sizeof(float));
-  if (!res) return MM_ERR_ALLOC_FAILED;
+  float *res = nullptr;
   if (is_pow2(n_fft)) {
     int st = gpu_available();
-    if (st != MM_OK) {
-      free(res);
-      return st;
-    }
+    if (st != MM_OK) return st;
     const size_t in_b = sizeof(float) * 2 * (size_t)n_freqs * n_frames;
     const size_t tw_b = sizeof(float2) * (size_t)n_fft, w_b = sizeof(float) * (size_t)n_fft;
     const size_t fr_b = sizeof(float) * (size_t)n_fft * n_frames, out_b = sizeof(float) * (size_t)out_len;
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t dev_b = up(in_b) + up(tw_b) + up(w_b) + up(fr_b) + up(out_b);
     Workspace *ws = nullptr;
-    if ((st = thread_workspace(dev_b, std::max(in_b, out_b), &ws)) != MM_OK) {
-      free(res);
-      return st;
-    }
+    if ((st = thread_workspace(dev_b, upload_staging(in_b), &ws)) != MM_OK) return st;
     cudaStream_t s = ws->stream;
     char *p = ws->dev;
     float2 *d_S = reinterpret_cast<float2 *>(p);
@@ -179,10 +172,7 @@ int32_t mm_istft(mm_context ctx, const float *stft_data, int64_t stft_count, int
     p += up(fr_b);
     float *d_out = reinterpret_cast<float *>(p);
     cudaError_t e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) {
-      memcpy(ws->host, stft_data, in_b);
-      e = cudaMemcpyAsync(d_S, ws->host, in_b, cudaMemcpyHostToDevice, s);
-    }
+    if (e == cudaSuccess) e = upload(reinterpret_cast<float *>(d_S), stft_data, in_b, ws);
     if (e == cudaSuccess) {
       istft_tables_kernel<<<(n_fft + 255) / 256, 256, 0, s>>>(d_tw, d_w, n_fft, win_length);
       e = cudaGetLastError();
@@ -202,14 +192,14 @@ int32_t mm_istft(mm_context ctx, const float *stft_data, int64_t stft_count, int
                                                    d_out);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ws->host, d_out, out_b, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
-      free(res);
       cudaGetLastError();
       return cuda_status(e);
     }
-    memcpy(res, ws->host, out_b);
+    if ((st = fetch_result(d_out, out_b, context_pooled(ctx), ws, &res)) != MM_OK) return st;
+  } else {
+    res = (float *)calloc((size_t)out_len, sizeof(float));
+    if (!res) return MM_ERR_ALLOC_FAILED;
   }
   out->data = res;
   out->shape[0] = out_len;

@@ -8,6 +8,8 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <unordered_map>
+#include <vector>
 
 namespace mm {
 
@@ -436,6 +438,129 @@ int thread_workspace(size_t dev_bytes, size_t host_bytes, Workspace **out) {
   }
   *out = &w;
   return MM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// host results
+// ---------------------------------------------------------------------------
+namespace {
+// Below kPoolMin the copies cost less than the bookkeeping; one block is at
+// most half of the cap, so that a result and the one before it both fit.
+constexpr size_t kPoolMin = size_t(256) << 10, kPoolCap = size_t(64) << 20;
+struct ResultPool {
+  std::mutex mu;
+  std::unordered_map<void *, size_t> live;  // handed out
+  std::multimap<size_t, void *> idle;
+  size_t total = 0;  // bytes of both
+  int refused = 0;   // requests since the last one that fitted
+};
+// never destroyed: results may be released while the process exits
+ResultPool &result_pool() {
+  static ResultPool *p = new ResultPool();
+  return *p;
+}
+// sizes are rounded up to a quarter of their power of two, so that calls on
+// clips of similar length share blocks
+size_t pool_class(size_t bytes) {
+  size_t step = kPoolMin / 4;
+  while (step * 8 < bytes) step *= 2;
+  return (bytes + step - 1) / step * step;
+}
+}  // namespace
+
+float *result_alloc(size_t bytes, bool pooled, bool *pinned) {
+  *pinned = false;
+  if (pooled && bytes >= kPoolMin && bytes <= kPoolCap / 2) {
+    ResultPool &rp = result_pool();
+    const size_t cls = pool_class(bytes);
+    std::vector<void *> drop;
+    bool fits = false;
+    {
+      std::lock_guard<std::mutex> lock(rp.mu);
+      auto it = rp.idle.find(cls);
+      if (it != rp.idle.end()) {
+        void *p = it->second;
+        rp.idle.erase(it);
+        rp.live[p] = cls;
+        rp.refused = 0;
+        *pinned = true;
+        return static_cast<float *>(p);
+      }
+      if (rp.total + cls > kPoolCap && ++rp.refused >= 16) {  // idle blocks of sizes no longer asked for
+        for (auto &b : rp.idle) {
+          rp.total -= b.first;
+          drop.push_back(b.second);
+        }
+        rp.idle.clear();
+        rp.refused = 0;
+      }
+      if (rp.total + cls <= kPoolCap) {
+        rp.total += cls;  // reserved while the block is made outside the lock
+        fits = true;
+      }
+    }
+    for (void *p : drop) cudaFreeHost(p);
+    if (fits) {
+      void *p = nullptr;
+      const cudaError_t e = cudaHostAlloc(&p, cls, cudaHostAllocPortable);
+      std::lock_guard<std::mutex> lock(rp.mu);
+      if (e == cudaSuccess) {
+        rp.live[p] = cls;
+        *pinned = true;
+        return static_cast<float *>(p);
+      }
+      cudaGetLastError();
+      rp.total -= cls;
+    }
+  }
+  return static_cast<float *>(malloc(bytes));
+}
+
+void result_free(void *p) {
+  if (!p) return;
+  ResultPool &rp = result_pool();
+  {
+    std::lock_guard<std::mutex> lock(rp.mu);
+    auto it = rp.live.find(p);
+    if (it != rp.live.end()) {
+      rp.idle.emplace(it->second, p);
+      rp.live.erase(it);
+      return;
+    }
+  }
+  free(p);
+}
+
+int fetch_result(const float *d, size_t bytes, bool pooled, Workspace *ws, float **out) {
+  bool pinned = false;
+  float *r = result_alloc(bytes, pooled, &pinned);
+  if (!r) return MM_ERR_ALLOC_FAILED;
+  cudaError_t e = cudaSuccess;
+  if (!pinned) {
+    Workspace *same = nullptr;
+    const int st = thread_workspace(0, bytes, &same);  // waits for the stream if the staging has to grow
+    if (st != MM_OK) {
+      result_free(r);
+      return st;
+    }
+  }
+  e = cudaMemcpyAsync(pinned ? reinterpret_cast<char *>(r) : ws->host, d, bytes, cudaMemcpyDeviceToHost, ws->stream);
+  const cudaError_t e2 = cudaStreamSynchronize(ws->stream);
+  if (e == cudaSuccess) e = e2;
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    result_free(r);
+    return cuda_status(e);
+  }
+  if (!pinned) memcpy(r, ws->host, bytes);
+  *out = r;
+  return MM_OK;
+}
+
+cudaError_t upload(float *d, const float *h, size_t bytes, Workspace *ws) {
+  if (bytes >= kDirectUpload) return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ws->stream);
+  memcpy(ws->host, h, bytes);
+  return cudaMemcpyAsync(d, ws->host, bytes, cudaMemcpyHostToDevice, ws->stream);
 }
 
 void fill_buffer(MMBuffer *out, float *data, long long rows, long long cols) {

@@ -132,36 +132,30 @@ int mel_dense(int sr, int n_fft, int n_mels, float fmin, float fmax, MelDense *o
 inline size_t up256(size_t v) { return (v + 255) & ~size_t(255); }
 
 // Host [n_rows, T] in, kernel(s) on the thread's stream, host [rows_out, T]
-// out (malloc'd, owned by the MMBuffer).
+// out (owned by the MMBuffer).
 template <typename Launch>
-int32_t run_columns(const float *S, int n_rows, long long T, int rows_out, size_t extra_dev, Launch launch,
+int32_t run_columns(mm_context ctx, const float *S, int n_rows, long long T, int rows_out, size_t extra_dev, Launch launch,
                     MMBuffer *out) {
   int st = gpu_available();
   if (st != MM_OK) return st;
   const size_t in_b = sizeof(float) * (size_t)n_rows * (size_t)T;
   const size_t out_b = sizeof(float) * (size_t)rows_out * (size_t)T;
   Workspace *ws = nullptr;
-  if ((st = thread_workspace(up256(in_b) + up256(out_b) + up256(extra_dev), std::max(in_b, out_b), &ws)) != MM_OK)
+  if ((st = thread_workspace(up256(in_b) + up256(out_b) + up256(extra_dev), upload_staging(in_b), &ws)) != MM_OK)
     return st;
   cudaStream_t s = ws->stream;
   float *d_in = reinterpret_cast<float *>(ws->dev);
   float *d_out = reinterpret_cast<float *>(ws->dev + up256(in_b));
   char *d_extra = ws->dev + up256(in_b) + up256(out_b);
   cudaError_t e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) {
-    memcpy(ws->host, S, in_b);
-    e = cudaMemcpyAsync(d_in, ws->host, in_b, cudaMemcpyHostToDevice, s);
-  }
+  if (e == cudaSuccess) e = upload(d_in, S, in_b, ws);
   if (e == cudaSuccess) e = launch(d_in, d_out, d_extra, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(ws->host, d_out, out_b, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return cuda_status(e);
   }
-  float *res = (float *)malloc(out_b > 0 ? out_b : 1);
-  if (!res) return MM_ERR_ALLOC_FAILED;
-  memcpy(res, ws->host, out_b);
+  float *res = nullptr;
+  if ((st = fetch_result(d_out, out_b, context_pooled(ctx), ws, &res)) != MM_OK) return st;
   fill_buffer(out, res, rows_out, T);
   return MM_OK;
 }
@@ -257,7 +251,7 @@ int32_t mm_mel_project(mm_context ctx, const float *S, int64_t count, int32_t n_
                                                                            d_out);
     return cudaGetLastError();
   };
-  return run_columns(S, n_freqs, T, n_mels, sizeof(int) * (size_t)T, launch, out);
+  return run_columns(ctx, S, n_freqs, T, n_mels, sizeof(int) * (size_t)T, launch, out);
 }
 
 // mfcc(S=...) on the GPU (feature.py:130-134 of the reference: scipy
@@ -281,7 +275,7 @@ int32_t mm_dct_ortho(mm_context ctx, const float *S, int64_t count, int32_t n_ro
     dct_cols_kernel<<<dim3(gx, (unsigned)rows_out), kColThreads, 0, s>>>(d_in, T, B, n_rows, d_out);
     return cudaGetLastError();
   };
-  return run_columns(S, n_rows, T, rows_out, sizeof(float) * (size_t)rows_out * n_rows, launch, out);
+  return run_columns(ctx, S, n_rows, T, rows_out, sizeof(float) * (size_t)rows_out * n_rows, launch, out);
 }
 
 // power_to_db of a device buffer on the caller's stream (asynchronous: the
