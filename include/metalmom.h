@@ -277,8 +277,8 @@ MM_API int32_t mm_plan_execute_host(mm_plan plan, const float* const* signals, f
 
 /* Autotuning of the frame kernel's launch variant, process-wide per n_fft:
  * variants 0-2 are the CTA-per-tile kernel with different frames per CTA and
- * register budgets; variant 3 (MFCC path, n_fft 256..2048) is the
- * frame-pair kernel (a warp pair per frame at 4096); variant 5 (MFCC path, n_fft 2048)
+ * register budgets; variant 3 (MFCC path, n_fft 256..4096) is the
+ * frame-pair kernel; variant 5 (MFCC path, n_fft 2048)
  * is the tensor-core kernel (both 32-point DFT stages as fp16x3 tcgen05
  * GEMMs).  mm_autotune times every variant that applies on n_clips synthetic
  * clips of clip_samples samples (reps launches each), writes each variant's

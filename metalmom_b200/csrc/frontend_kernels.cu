@@ -1263,7 +1263,7 @@ cudaError_t launch_frontend(int log2n, int mode, int variant, const FrontArgs &a
       if (pw != 0) return cudaErrorInvalidValue;
       if (variant == kTcVariant && log2n == 11) return launch_frontend_tc(a, grid_limit, s, launched);
       if (variant == kWarpVariant && warp_frames_per_tile(log2n) > 0)
-        return launch_frontend_warp(log2n, a, grid_limit, s, launched);
+        return launch_frontend_pair(log2n, a, grid_limit, s, launched);
       return launch_mode<MODE_MELDB, 0>(log2n, variant, a, grid_limit, s, launched);
     default: return cudaErrorInvalidValue;
   }

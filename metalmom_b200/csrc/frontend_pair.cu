@@ -1,4 +1,4 @@
-// Frame-pair front-end kernel (launch variant 3, n_fft 256..2048, MFCC path):
+// Frame-pair front-end kernels (launch variant 3, n_fft 256..4096, MFCC path):
 // framing + periodic Hann + real FFT + |X|^2 + Slaney mel + log10, two
 // consecutive frames per group of lanes, with a running per-clip maximum for
 // top_db.
@@ -21,8 +21,9 @@
 //   pair (Z[k], Z[M-k]): the stage-2 columns are dealt to lanes so that k1
 //   and 32-k1 sit in the same lane (TPF < 32); for TPF = 32 the partner lanes
 //   l and 32-l swap the upper 16 registers by shuffle and each takes 16 pairs.
+// n_fft 4096 has 64 lanes, a warp pair (frame_pair4096_kernel below).
 //
-// Only warp-level synchronisation is used.  The window is staged in shared
+// Only warp-level (4096: warp-pair) synchronisation is used.  The window is staged in shared
 // memory halved (exact in binary floating point), so the real split's
 // E + W O, formed without its factor 1/2, is X itself and the spectrum is
 // |X|^2, bit for bit the values of the unscaled transform divided by 4: a bin
@@ -39,7 +40,8 @@
 // the kernel now waits on its own latencies (issue 44 %, shared-memory pipe
 // 67 %).  256 clips of 30 s at n_fft 2048, hop 512, 128 bands: 0.90 -> 0.77 ms
 // (whole step 0.954 -> 0.833); 512 clips of 10 s at n_fft 512, hop 160, 80
-// bands: 0.46 ms against 0.62 for the CTA-tile kernel (whole step 0.431).
+// bands, whole step: 0.62 (CTA-tile kernel) -> 0.42.  64 clips of 30 s at 44.1 kHz,
+// n_fft 4096, hop 1024: 0.571 -> 0.511 (one frame per warp pair, 16 warps, before).
 // Measured and left out (128 clips, whole step, against 0.426 ms): 12 warps of
 // 168 registers 0.443; the next pair's samples loaded into registers before
 // the walk 0.445 against 0.438; the next pair's 16-point DFTs interleaved with
@@ -56,6 +58,9 @@
 
 namespace mm {
 
+// Float pairs per 32 bins of a pair's spectrum: 34, so that a lane's bins are
+// 16-byte aligned; 33 for a warp pair, whose store pattern needs it odd.
+__host__ __device__ constexpr int pair_ps(int tpf) { return tpf == 64 ? 33 : 34; }
 constexpr float k10Log10of2 = 3.0102999566398120f;  // 10 log10(2)
 
 template <int LOG2N>
@@ -76,7 +81,7 @@ struct PShape {
   // of row j swapped within groups of 8 by XOR with j mod 8 (both ways of
   // access conflict-free)
   static constexpr int BS = TPF == 32 ? 1024 : TPF * 33 + (TPF == 8 ? 16 : 0);
-  static constexpr int PS = 34;  // float pairs per 32 bins of the spectrum
+  static constexpr int PS = pair_ps(TPF);
   static_assert(TPF >= 4 && TPF <= 32, "n_fft must be 256..2048");
 };
 
@@ -98,13 +103,27 @@ __host__ __device__ constexpr size_t pair_warp_smem() {
   return size_t(PShape<LOG2N>::FPW) * PShape<LOG2N>::BS * 16;
 }
 
+// n_fft 4096: a pair of frames on a warp pair (frame_pair4096_kernel)
+struct P4Shape {
+  static constexpr int N = 4096, M = N / 2, TPF = 64;
+  static constexpr int NP = 4;  // warp pairs per CTA, one CTA per SM
+  static constexpr int UF = 2, UT = 4;
+  static constexpr int BS = TPF * 33;  // 16-byte slots of a buffer
+  static constexpr int PS = pair_ps(TPF);
+  static constexpr int RS = 16 * 33;   // real-split factors, rows of 33
+  static constexpr int MEL_SMEM_MAX = 1024;
+  static constexpr size_t fixed = size_t(16) * TPF * 16 + size_t(N) * 4 + size_t(RS) * 16;
+  static constexpr size_t walk = (16 * 24 + 16) * size_t(TPF);
+  static_assert(PS * TPF * 8 % 16 == 0 && PS * TPF / 2 + 1024 <= BS, "spectrum and 1 024 parts fit the buffer");
+};
+
 int warp_frames_per_tile(int log2n) {
   switch (log2n) {
     case 8: return PShape<8>::F;
     case 9: return PShape<9>::F;
     case 10: return PShape<10>::F;
     case 11: return PShape<11>::F;
-    case 12: return 8;  // frame_warp2_kernel: one frame per warp pair, 16 warps
+    case 12: return P4Shape::UF * P4Shape::UT;
     default: return 0;
   }
 }
@@ -168,8 +187,332 @@ __device__ __forceinline__ void walk_end(f2 p, float wr, float wf, unsigned fl, 
 template <int TPF>
 __device__ __forceinline__ int pair_bin(int k) {
   const int q = k >> 5;
-  return k + 2 * (q < TPF - 1 ? q : TPF - 1);
+  return k + (pair_ps(TPF) - 32) * (q < TPF - 1 ? q : TPF - 1);
 }
+
+// Synchronisation of the lanes that own a pair: part of a warp (any() of the
+// lanes in `mask`), or the 64 threads of a warp pair on named barrier id + 1.
+struct GroupSync {
+  unsigned mask;
+  __device__ __forceinline__ void operator()() const { __syncwarp(); }
+  __device__ __forceinline__ bool any(bool p) const { return (__ballot_sync(0xffffffffu, p) & mask) != 0; }
+};
+struct WarpPairSync {
+  int id;
+  __device__ __forceinline__ void operator()() const { frame_sync<64>(id); }
+  __device__ __forceinline__ bool any(bool p) const { return frame_sync_or<64>(id, p); }
+};
+
+// Tables of the filterbank walk (walk_bands) in shared memory.
+struct WalkTables {
+  const float4 *wa;   // [16][TPF]
+  const float2 *wb;   // [16][TPF]
+  const int4 *lane;   // [TPF]
+  const int *band;
+  bool twice;         // some pair of bins ends two segments
+};
+
+// Stages them from the lane tables (build_mel_lane_kernel), lane-minor: per
+// pair of bins g < 16 of lane l the weights (rising, falling) of the first bin
+// and of the second in the segment that is open (wa), and of the second in a
+// segment it starts (wb); and the lane words.  True when this thread saw a
+// pair of bins that ends two segments.
+template <int TPF>
+__device__ __forceinline__ bool stage_walk(const FrontArgs &a, float4 *wa, float2 *wb, int4 *lane_s, int tid,
+                                           int threads) {
+  bool twice = false;
+  // flush bits of a lane's bins, bin 31 left to the end of the walk
+  auto flush_bit = [&](int2 w, int bin) { return bin < 31 ? ((unsigned)w.x >> bin) & 1u : 0u; };
+  for (int i = tid; i < TPF; i += threads) {
+    const int2 w = __ldg(a.mel_lane + i);
+    unsigned m1 = 0u, m2 = 0u;
+    for (int g = 0; g < 16; g++) {
+      const unsigned fa = flush_bit(w, 2 * g), fb = flush_bit(w, 2 * g + 1);
+      m1 |= (fa | fb) << g;
+      m2 |= (fa & fb) << g;
+    }
+    // {first | second segment end by pair, first part's byte offset, parts the
+    // head takes over from the next lanes, the empty segments' slot}
+    lane_s[i] = make_int4((int)(m1 | m2 << 16), 16 * (w.y & 1023), (w.y >> 10) & 63, w.y >> 16);
+    if (m2) twice = true;
+  }
+  for (int i = tid; i < 16 * TPF; i += threads) {
+    const int g = i / TPF, j = i - g * TPF;
+    const bool fa = flush_bit(__ldg(a.mel_lane + j), 2 * g) != 0;
+    const float2 u = __ldg(a.mel_lw + 2 * g * TPF + j), w = __ldg(a.mel_lw + (2 * g + 1) * TPF + j);
+    wa[i] = make_float4(u.x, u.y, fa ? 0.0f : w.x, fa ? 0.0f : w.y);
+    wb[i] = make_float2(fa ? w.x : 0.0f, fa ? w.y : 0.0f);
+  }
+  return twice;
+}
+
+// A band's dB value of both frames into their rows, and the running maximum.
+__device__ __forceinline__ void put_band(const FrontArgs &a, f2 sum, int m, float ref_db, float *dst, bool va, bool vb,
+                                         float &vmax) {
+  float xa, xb;
+  un2(sum, xa, xb);
+  const float da = fmaf(k10Log10of2, __log2f(fmaxf(xa, a.amin)), -ref_db);
+  const float db = fmaf(k10Log10of2, __log2f(fmaxf(xb, a.amin)), -ref_db);
+  if (va) {
+    dst[m] = da;
+    vmax = fmaxf(vmax, da);
+  }
+  if (vb) {
+    dst[a.n_mels + m] = db;
+    vmax = fmaxf(vmax, db);
+  }
+}
+
+// The filterbank walk.  Lane l sums its 32 bins (the last lane also the
+// Nyquist bin) into (R, F) = (rising, falling weight) times P and stores the
+// sums in the next part slot at every segment end.  Bins go in pairs: the
+// second bin of a pair has its weights in one of two sets, zero in the other,
+// wa.zw for the segment that the first bin belongs to and wb for a segment
+// that it starts, so one predicated store and restart serve a pair wherever in
+// it the segment ends.  Pairs that end two segments (bands of a single bin)
+// take the second end in a branch of their own.
+template <int TPF, typename Sync>
+__device__ __forceinline__ void walk_bands(const FrontArgs &a, const Sync &sync, const f2 *P, cpx2 *parts, int l,
+                                           const WalkTables &w, float ref_db, float *dst, bool va, bool vb,
+                                           float &vmax) {
+  const int4 li = w.lane[l];
+  const unsigned fl = (unsigned)li.x;
+  const uint32_t part0 = smem_u32(parts);
+  uint32_t at = part0 + (unsigned)li.y;  // the next part's slot
+  const f2 *pl = P + pair_ps(TPF) * l;
+  auto bins = [&](int g) {  // bins 2g, 2g + 1 of both frames
+    if constexpr (pair_ps(TPF) % 2 == 0) return reinterpret_cast<const float4 *>(pl)[g];
+    else return make_float4(lo2(pl[2 * g]), hi2(pl[2 * g]), lo2(pl[2 * g + 1]), hi2(pl[2 * g + 1]));
+  };
+  const float4 *wa = w.wa + l;
+  const float2 *wb = w.wb + l;
+  const f2 zero = dup2(0.0f);
+  f2 R = zero, Fs = zero;
+  // the frames' non-finite check: the largest bit pattern of a power (a power
+  // is never negative; NaN and inf lie at or above inf's pattern)
+  unsigned mxa = 0u, mxb = 0u;
+  static_for<0, 16>([&](auto gi) {
+    constexpr int g = decltype(gi)::value;
+    const float4 pq = bins(g), u = wa[g * TPF];
+    const float2 v = wb[g * TPF];
+    mxa = max(max(mxa, __float_as_uint(pq.x)), __float_as_uint(pq.z));
+    mxb = max(max(mxb, __float_as_uint(pq.y)), __float_as_uint(pq.w));
+    const f2 p0 = pk2(pq.x, pq.y), p1 = pk2(pq.z, pq.w);
+    R = fma2(p0, dup2(u.x), R);
+    Fs = fma2(p0, dup2(u.y), Fs);
+    R = fma2(p1, dup2(u.z), R);
+    Fs = fma2(p1, dup2(u.w), Fs);
+    walk_end<g>(p1, v.x, v.y, fl, R, Fs, at);
+    if (w.twice && (fl & (0x10000u << g))) {
+      walk_store(at, R, Fs);
+      at += 16;
+      R = zero;
+      Fs = zero;
+    }
+  });
+  if (l == TPF - 1) {
+    if (__ldg(a.mel_lane + l).x < 0) {  // bin 31 ends a segment
+      walk_store(at, R, Fs);
+      at += 16;
+      R = zero;
+      Fs = zero;
+    }
+    float pa, pb2;
+    un2(pl[32], pa, pb2);
+    const float2 wn = __ldg(a.mel_lw + 32 * TPF + l);
+    mxa = max(mxa, __float_as_uint(pa));
+    mxb = max(mxb, __float_as_uint(pb2));
+    R = fma2(pl[32], dup2(wn.x), R);
+    Fs = fma2(pl[32], dup2(wn.y), Fs);
+  }
+  walk_store(at, R, Fs);
+  if (l == 0) parts[li.w] = {zero, zero};  // the empty segments' slot
+  const bool bada = sync.any(mxa >= 0x7f800000u), badb = sync.any(mxb >= 0x7f800000u);
+  // added to a frame's band sums: NaN where a bin of it is not finite
+  const float qnan = __int_as_float(0x7fc00000);
+  const f2 nan2 = pk2(bada ? qnan : 0.0f, badb ? qnan : 0.0f);
+  sync();
+  // a lane whose last part heads a segment adds the parts of the lanes the
+  // segment runs into
+  if (li.z) {
+    cpx2 *h = parts + ((at - part0) >> 4);
+    cpx2 hv = *h;
+    for (int j = 1; j <= li.z; j++) hv = cadd(hv, h[j]);
+    *h = hv;
+  }
+  sync();
+  // band m is the head of segment m (rising) plus the head of segment m + 1
+  // (falling); four bands at a time, so that their reads overlap.  The lane
+  // tables hold finite weights only: no band is NaN by itself.
+  const char *pb = reinterpret_cast<const char *>(parts);
+  for (int m0 = l; m0 < a.n_mels; m0 += 4 * TPF) {
+    int bw[4];
+    f2 acc[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) bw[i] = m0 + i * TPF < a.n_mels ? w.band[m0 + i * TPF] : 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      acc[i] = add2(*reinterpret_cast<const f2 *>(pb + 16 * (bw[i] & 4095)),
+                    *reinterpret_cast<const f2 *>(pb + 8 + 16 * ((bw[i] >> 12) & 4095)));
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int m = m0 + i * TPF;
+      put_band(a, add2(acc[i], nan2), m, ref_db, dst, va && m < a.n_mels, vb && m < a.n_mels, vmax);
+    }
+  }
+}
+
+// The bands of a filterbank that the lane tables cannot describe, from packed rows.
+template <int TPF, typename Sync>
+__device__ __forceinline__ void row_bands(const FrontArgs &a, const Sync &sync, const f2 *P, int l, const float *melw,
+                                          float ref_db, float *dst, bool va, bool vb, float &vmax) {
+  unsigned mxa = 0u, mxb = 0u;  // the non-finite check: this lane's share of the bins
+  for (int k = l; k <= 32 * TPF; k += TPF) {
+    float pa, pb;
+    un2(P[pair_bin<TPF>(k)], pa, pb);
+    mxa = max(mxa, __float_as_uint(pa));
+    mxb = max(mxb, __float_as_uint(pb));
+  }
+  const bool bada = sync.any(mxa >= 0x7f800000u), badb = sync.any(mxb >= 0x7f800000u);
+  const float qnan = __int_as_float(0x7fc00000);
+  for (int m = l; m < a.n_mels; m += TPF) {
+    const int4 info = __ldg(a.mel_info + m);
+    const float *wr = melw + info.z;
+    f2 acc = dup2(0.0f);
+    for (int q = 0; q < info.y; q++) acc = fma2(P[pair_bin<TPF>(info.x + q)], dup2(wr[q]), acc);
+    acc = add2(acc, pk2(info.w || bada ? qnan : 0.0f, info.w || badb ? qnan : 0.0f));
+    put_band(a, acc, m, ref_db, dst, va, vb, vmax);
+  }
+}
+
+// Samples (x[2n], x[2n+1]), n = l + TPF r, r < n_q, of the frame that starts at
+// s0 (and, with the overlap of the next, `reach` samples more).
+template <int TPF, bool EVEN, int NQ>
+__device__ __forceinline__ void gather_frame(float2 (&q)[NQ], const FrontArgs &a, const ClipDesc &cd, long long s0,
+                                             int reach, int l) {
+  const float *base = a.signal + cd.sig_off + s0 + 2 * l;
+  if (s0 >= 0 && s0 + reach + 64 * TPF <= cd.length) {
+    if (EVEN || ((cd.sig_off + s0) & 1) == 0) {
+#pragma unroll
+      for (int r = 0; r < NQ; r++) q[r] = __ldg(reinterpret_cast<const float2 *>(base + 2 * TPF * r));
+    } else {
+#pragma unroll
+      for (int r = 0; r < NQ; r++) q[r] = make_float2(__ldg(base + 2 * TPF * r), __ldg(base + 2 * TPF * r + 1));
+    }
+  } else {  // frames that reach into the padding (a few per clip)
+    float2 te[NQ];
+    gather_edge_n<NQ>(te, a.signal + cd.sig_off, s0 + 2 * l, cd.length, a.pad_mode, 2 * TPF);
+#pragma unroll
+    for (int r = 0; r < NQ; r++) q[r] = te[r];
+  }
+}
+
+// Both frames times the window; even registers into e, odd ones into o.
+template <int TPF>
+__device__ __forceinline__ void window_pair(const float2 *qa, const float2 *qb, const float4 *wl, cpx2 *e, cpx2 *o) {
+#pragma unroll
+  for (int r = 0; r < 32; r += 2) {
+    const float4 w = wl[TPF * (r / 2)];
+    e[r / 2] = {pk2(qa[r].x * w.x, qb[r].x * w.x), pk2(qa[r].y * w.y, qb[r].y * w.y)};
+    o[r / 2] = {pk2(qa[r + 1].x * w.z, qb[r + 1].x * w.z), pk2(qa[r + 1].y * w.w, qb[r + 1].y * w.w)};
+  }
+}
+
+// Frames t and t + 1 gathered and windowed (D: see frame_pair_kernel).
+template <int TPF, int D>
+__device__ __forceinline__ void load_pair(const FrontArgs &a, const ClipDesc &cd, int t, int l, const float4 *win_s,
+                                          cpx2 *e, cpx2 *o) {
+  const long long s0 = (long long)t * a.hop - a.pad;
+  float2 q[D > 0 ? 32 + D : 32];
+  gather_frame<TPF, (D > 0)>(q, a, cd, s0, D > 0 ? a.hop : 0, l);
+  if constexpr (D > 0) {
+    window_pair<TPF>(q, q + D, win_s + l, e, o);
+  } else {
+    float2 qb[32];
+    gather_frame<TPF, false>(qb, a, cd, s0 + a.hop, 0, l);
+    window_pair<TPF>(q, qb, win_s + l, e, o);
+  }
+}
+
+// The last butterflies of a pair's stage 1 (e, o: its two 16-point DFTs), each
+// followed by the twiddle W_M^(j k1) of row j (tw at [k TPF]) and put(k1, value).
+template <int TPF, typename Put>
+__device__ __forceinline__ void finish_stage1(const cpx2 *e, const cpx2 *o, const float4 *tw, Put &&put) {
+  static_for<0, 16>([&](auto ki) {
+    constexpr int k = decltype(ki)::value;
+    using R = Rot<k, 32>;
+    cpx2 lo, hi;
+    rot_butterfly<R>(e[k], R::rot(o[k]), lo, hi);
+    const float4 tk = tw[k * TPF];
+    if constexpr (k > 0) lo = cmul(lo, {tk.x, tk.y});
+    hi = cmul(hi, {tk.z, tk.w});
+    put(std::integral_constant<int, k>{}, lo);
+    put(std::integral_constant<int, k + 16>{}, hi);
+  });
+}
+
+// |X[k]|^2 and |X[M-k]|^2 of both frames from za = Z[k], zb = Z[M-k] and the
+// factors (scale, ratio) of W_N^k: (cos, tan) below an eighth of a turn (LOW),
+// (sin, cot) above.  The window was halved.
+template <bool LOW>
+__device__ __forceinline__ void split_pair(cpx2 za, cpx2 zb, float scale, float ratio, f2 &p, f2 &q) {
+  const f2 ex = add2(za.x, zb.x), ey = sub2(za.y, zb.y);
+  const f2 ox = add2(za.y, zb.y), oy = sub2(zb.x, za.x);
+  const f2 sc = dup2(scale), rt = dup2(ratio);
+  f2 wr, wi;  // W_N^k O without its scale
+  if constexpr (LOW) {
+    wr = fma2(oy, rt, ox);
+    wi = fma2(neg2(ox), rt, oy);
+  } else {
+    wr = fma2(ox, rt, oy);
+    wi = fma2(oy, rt, neg2(ox));
+  }
+  const f2 xr = fma2(wr, sc, ex), xi = fma2(wi, sc, ey);
+  const f2 yr = fma2(neg2(wr), sc, ex), yi = fma2(neg2(wi), sc, ey);
+  p = fma2(xr, xr, mul2(xi, xi));
+  q = fma2(yr, yr, mul2(yi, yi));
+}
+
+// The factors of split_pair for W_N^k = c - i s as (scale, ratio).
+__device__ __forceinline__ float2 split_factors(cpx w, bool low) {
+  return low ? make_float2(w.x, -w.y / w.x) : make_float2(-w.y, w.x / -w.y);
+}
+
+// The warp's running maximum of clip `clip` into its slot.
+__device__ __forceinline__ void flush_max(const FrontArgs &a, int clip, float vmax, int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+  if (lane == 0 && clip >= 0 && vmax > -INFINITY) atomicMax(a.clip_max + clip, enc_f(vmax));
+}
+
+// The units of work of one warp (or warp pair): `first`, then every `step`-th
+// of this CTA's contiguous range that holds a frame.
+template <int UF, int UT>
+struct Units {
+  int u, end, step;
+  int clip = -1, past = -1;  // past: first unit after the current clip
+  ClipDesc cd{};
+  // A CTA's range is dealt to its warps in turn, so that the samples its warps
+  // read at a time overlap.
+  __device__ __forceinline__ Units(const FrontArgs &a, int worker, int workers) {
+    const long long total = (long long)a.total_tiles * UT;
+    u = (int)(blockIdx.x * total / gridDim.x) + worker - workers;
+    end = (int)((blockIdx.x + 1) * total / gridDim.x);
+    step = workers;
+  }
+  __device__ __forceinline__ int first_frame() const { return (u - cd.tile_base * UT) * UF; }
+  __device__ __forceinline__ bool advance(const FrontArgs &a) {
+    while ((u += step) < end) {
+      if (u >= past) {  // every frame of a tile belongs to one clip
+        clip = __ldg(a.tile_clip + u / UT);
+        cd = load_clip(a.clips + clip);
+        past = (cd.tile_base + (cd.n_frames + UF * UT - 1) / (UF * UT)) * UT;
+      }
+      if (first_frame() < cd.n_frames) return true;
+    }
+    return false;
+  }
+};
 
 // D > 0: hop = 2 TPF D samples and every clip starts at an even sample, so
 // register r of frame t + 1 is register r + D of frame t and the pair's gather
@@ -235,35 +578,11 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
     for (int i = tid; i < 8 * 32; i += threads) {
       const int p = i >> 5, ll = i & 31;
       const cpx u = root_q(twq, ll + 64 * p, N), w = root_q(twq, ll + 32 * (2 * p + 1), N);
-      // W = c - i s: both entries of p lie on the same side of an eighth of a turn
-      rs_tw[i] = p < 4 ? make_float4(u.x, -u.y / u.x, w.x, -w.y / w.x)
-                       : make_float4(-u.y, u.x / -u.y, -w.y, w.x / -w.y);
+      // both entries of p lie on the same side of an eighth of a turn
+      const float2 fu = split_factors(u, p < 4), fw = split_factors(w, p < 4);
+      rs_tw[i] = make_float4(fu.x, fu.y, fw.x, fw.y);
     }
-  bool twice = false;  // some pair of bins ends two segments
-  if (lanes) {
-    // flush bits of a lane's bins, bin 31 left to the end of the walk
-    auto flush_bit = [&](int2 w, int bin) { return bin < 31 ? ((unsigned)w.x >> bin) & 1u : 0u; };
-    for (int i = tid; i < TPF; i += threads) {
-      const int2 w = __ldg(a.mel_lane + i);
-      unsigned m1 = 0u, m2 = 0u;
-      for (int g = 0; g < 16; g++) {
-        const unsigned fa = flush_bit(w, 2 * g), fb = flush_bit(w, 2 * g + 1);
-        m1 |= (fa | fb) << g;
-        m2 |= (fa & fb) << g;
-      }
-      // {first | second segment ends by pair, first part's byte offset, parts
-      // the head takes over from the next lanes, the empty segments' slot}
-      lane_s[i] = make_int4((int)(m1 | m2 << 16), 16 * (w.y & 1023), (w.y >> 10) & 63, w.y >> 16);
-      if (m2) twice = true;
-    }
-    for (int i = tid; i < 16 * TPF; i += threads) {
-      const int g = i / TPF, j = i - g * TPF;
-      const bool fa = flush_bit(__ldg(a.mel_lane + j), 2 * g) != 0;
-      const float2 u = __ldg(a.mel_lw + 2 * g * TPF + j), w = __ldg(a.mel_lw + (2 * g + 1) * TPF + j);
-      wa_s[i] = make_float4(u.x, u.y, fa ? 0.0f : w.x, fa ? 0.0f : w.y);
-      wb_s[i] = make_float2(fa ? w.x : 0.0f, fa ? w.y : 0.0f);
-    }
-  }
+  bool twice = lanes && stage_walk<TPF>(a, wa_s, wb_s, lane_s, tid, threads);
   const int *src_words = lanes ? a.mel_band : reinterpret_cast<const int *>(a.mel_pw);
   if (staged)
     for (int i = tid; i < words; i += threads) words_s[i] = __ldg(src_words + i);
@@ -290,93 +609,24 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
   // so that the two groups of a half warp store to disjoint banks
   f2 *P = reinterpret_cast<f2 *>(fb) + (TPF == 8 ? 8 * grp : 0);
   cpx2 *parts = reinterpret_cast<cpx2 *>(P + PS * TPF);  // {R, F} of both frames per part
-  const unsigned gmask = (TPF == 32) ? FULL : (((1u << TPF) - 1u) << (grp * TPF));
+  const GroupSync sync{(TPF == 32) ? FULL : (((1u << TPF) - 1u) << (grp * TPF))};
 
-  // This CTA's units (2 FPW consecutive frames of one clip each) are a
-  // contiguous range dealt to its warps in turn, so that the samples its
-  // warps read at a time overlap.
-  const long long total = (long long)a.total_tiles * S::UT;
-  const int u_end = (int)((blockIdx.x + 1) * total / gridDim.x);
-  int cur = -1, next_clip = -1;  // next_clip: first unit past the current clip
-  ClipDesc cd{};
+  Units<S::UF, S::UT> units(a, warp, nw);  // 2 FPW consecutive frames of one clip each
   int vclip = -1;  // the clip vmax belongs to
   float vmax = -INFINITY;
-
-  // Moves on to this warp's next unit with a frame in it; false at the end.
-  int u = (int)(blockIdx.x * total / gridDim.x) + warp - nw;
-  auto advance = [&]() {
-    while ((u += nw) < u_end) {
-      if (u >= next_clip) {  // warp-uniform: every frame of a tile belongs to one clip
-        cur = __ldg(a.tile_clip + u / S::UT);
-        cd = load_clip(a.clips + cur);
-        next_clip = (cd.tile_base + (cd.n_frames + S::F - 1) / S::F) * S::UT;
-      }
-      if ((u - cd.tile_base * S::UT) * S::UF < cd.n_frames) return true;
-    }
-    return false;
-  };
-  auto first_frame = [&]() { return (u - cd.tile_base * S::UT) * S::UF + 2 * grp; };
-
-  // Raw samples (x[2n], x[2n+1]), n = l + TPF r, of this warp's next unit:
-  // register r of frame t, and with D > 0 of frame t + 1 at r + D.
-  constexpr int Q = D > 0 ? 32 + D : 32;
-  auto gather_frame = [&](auto &dst_q, int t, int reach) {
-    constexpr int n = sizeof(dst_q) / sizeof(float2);
-    const long long s0 = (long long)t * a.hop - a.pad;
-    const float *base = a.signal + cd.sig_off + s0 + 2 * l;
-    if (s0 >= 0 && s0 + reach + N <= cd.length) {
-      if (D > 0 || ((cd.sig_off + s0) & 1) == 0) {
-#pragma unroll
-        for (int r = 0; r < n; r++) dst_q[r] = __ldg(reinterpret_cast<const float2 *>(base + 2 * TPF * r));
-      } else {
-#pragma unroll
-        for (int r = 0; r < n; r++)
-          dst_q[r] = make_float2(__ldg(base + 2 * TPF * r), __ldg(base + 2 * TPF * r + 1));
-      }
-    } else {  // frames that reach into the padding (a few per clip)
-      float2 te[n];
-      gather_edge_n<n>(te, a.signal + cd.sig_off, s0 + 2 * l, cd.length, a.pad_mode, 2 * TPF);
-#pragma unroll
-      for (int r = 0; r < n; r++) dst_q[r] = te[r];
-    }
-  };
-  // window; even registers into e, odd ones into o
-  auto window = [&](const float2 *qa, const float2 *qb, cpx2 *e, cpx2 *o) {
-    const float4 *wb = win_s + l;
-#pragma unroll
-    for (int r = 0; r < 32; r += 2) {
-      const float4 w = wb[TPF * (r / 2)];
-      e[r / 2] = {pk2(qa[r].x * w.x, qb[r].x * w.x), pk2(qa[r].y * w.y, qb[r].y * w.y)};
-      o[r / 2] = {pk2(qa[r + 1].x * w.z, qb[r + 1].x * w.z), pk2(qa[r + 1].y * w.w, qb[r + 1].y * w.w)};
-    }
-  };
-
-  bool more = advance();
-  while (more) {
-    if (cur != vclip) {
-      float m = vmax;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-      if (lane == 0 && vclip >= 0 && m > -INFINITY) atomicMax(a.clip_max + vclip, enc_f(m));
-      vclip = cur;
+  while (units.advance(a)) {
+    if (units.clip != vclip) {
+      flush_max(a, vclip, vmax, lane);
+      vclip = units.clip;
       vmax = -INFINITY;
     }
-    const int tw0 = first_frame() - 2 * grp, t = tw0 + 2 * grp;
+    const ClipDesc &cd = units.cd;
+    const int tw0 = units.first_frame(), t = tw0 + 2 * grp;
     const bool va = t < cd.n_frames, vb = t + 1 < cd.n_frames;
     float *dst = a.out + (cd.frame_off + t) * (long long)nmel;
 
     cpx2 e[16], o[16];
-    {
-      float2 q[Q];
-      gather_frame(q, t, D > 0 ? a.hop : 0);
-      if constexpr (D > 0) {
-        window(q, q + D, e, o);
-      } else {
-        float2 qb[32];
-        gather_frame(qb, t + 1, 0);
-        window(q, qb, e, o);
-      }
-    }
+    load_pair<TPF, D>(a, cd, t, l, win_s, e, o);
     // the samples that this warp's next unit adds to the CTA's, into L1: one
     // line a lane (n_fft 1024: 0.459 against 0.466 ms for 128 clips of 30 s)
     {
@@ -392,21 +642,10 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
     __syncwarp();  // the previous unit's reads of the buffer are done
     {
       cpx2 *row = fb + l * (TPF == 32 ? 32 : 33);
-      static_for<0, 16>([&](auto ki) {
+      finish_stage1<TPF>(e, o, tw4 + l, [&](auto ki, cpx2 y) {
         constexpr int k = decltype(ki)::value;
-        using R = Rot<k, 32>;
-        cpx2 lo, hi;
-        rot_butterfly<R>(e[k], R::rot(o[k]), lo, hi);
-        const float4 tk = tw4[k * TPF + l];
-        if constexpr (k > 0) lo = cmul(lo, {tk.x, tk.y});
-        hi = cmul(hi, {tk.z, tk.w});
-        if constexpr (TPF == 32) {
-          row[(k & 8) + ((k & 7) ^ (l & 7))] = lo;
-          row[16 + (k & 8) + ((k & 7) ^ (l & 7))] = hi;
-        } else {
-          row[k] = lo;
-          row[k + 16] = hi;
-        }
+        if constexpr (TPF == 32) row[(k & 24) + ((k & 7) ^ (l & 7))] = y;
+        else row[k] = y;
       });
     }
     __syncwarp();
@@ -443,21 +682,9 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
         const cpx2 rcv = {shfl2(up.x, src), shfl2(up.y, src)};
         const cpx2 zb = csel(l0, prev, rcv);
         prev = up;
-        const f2 ex = add2(za.x, zb.x), ey = sub2(za.y, zb.y);
-        const f2 ox = add2(za.y, zb.y), oy = sub2(zb.x, za.x);
         if constexpr (i % 2 == 0) rsp = rs_tw[32 * (i / 2) + l];
-        const f2 sc = dup2(i % 2 == 0 ? rsp.x : rsp.z), rt = dup2(i % 2 == 0 ? rsp.y : rsp.w);
-        f2 wr, wi;  // W_N^(l + 32 i) O without its scale
-        if constexpr (i < 8) {
-          wr = fma2(oy, rt, ox);
-          wi = fma2(neg2(ox), rt, oy);
-        } else {
-          wr = fma2(ox, rt, oy);
-          wi = fma2(oy, rt, neg2(ox));
-        }
-        const f2 xr = fma2(wr, sc, ex), xi = fma2(wi, sc, ey);
-        const f2 yr = fma2(neg2(wr), sc, ex), yi = fma2(neg2(wi), sc, ey);
-        const f2 p = fma2(xr, xr, mul2(xi, xi)), q = fma2(yr, yr, mul2(yi, yi));
+        f2 p, q;
+        split_pair<(i < 8)>(za, zb, i % 2 == 0 ? rsp.x : rsp.z, i % 2 == 0 ? rsp.y : rsp.w, p, q);
         Pa[PS * i] = p;
         if constexpr (i == 0) Pb[l0 ? -2 : 0] = q;  // lane 0: the Nyquist bin
         else Pb[-PS * i] = q;
@@ -510,144 +737,180 @@ __global__ void __launch_bounds__(32 * PShape<LOG2N>::NW, 1) frame_pair_kernel(F
     }
     __syncwarp();  // P complete
 
-    more = advance();
+    // ---- log-mel rows of both frames + running clip max
+    if (lanes) walk_bands<TPF>(a, sync, P, parts, l, {wa_s, wb_s, lane_s, band, twice}, ref_db, dst, va, vb, vmax);
+    else row_bands<TPF>(a, sync, P, l, melw, ref_db, dst, va, vb, vmax);
+  }
+  flush_max(a, vclip, vmax, lane);
+}
+
+// ---------------------------------------------------------------------------
+// n_fft 4096: a pair of frames on a warp pair (64 threads), the same work.
+//
+//   n = j + 64 r (j < 64: thread of the pair, r < 32), k = k1 + 32 k2 (k2 < 64)
+//   stage 1: 32-point DFT over r in registers, twiddle W_M^(j k1), row j of
+//            the buffer (16-byte elements, stride 33)
+//   stage 2: the 64-point DFT over j of column k1 as 2 x 32: thread (k1, j0)
+//            takes rows j0 + 2 j1 (j1 < 32) through a 32-point DFT -> A_j0[q];
+//            the two threads of a column (lanes 2i, 2i+1) swap half of their
+//            outputs by shuffle, and thread j0 forms
+//            Z[k1 + 32 q] = A_0[q] + W_64^q A_1[q] and
+//            Z[k1 + 32 (q + 32)] = A_0[q] - W_64^q A_1[q] for q = 2 i + j0.
+//   Even columns live in the pair's first warp, odd ones in its second
+//   (lane = 2 (k1 >> 1) + j0), so the real-split partner (32 - k1, 1 - j0)
+//   of a thread sits in its warp; the two swap their upper 16 registers by
+//   shuffle.  Column 0 pairs inside each thread.
+// Every shared-memory pattern (row stores, column loads, twiddles, spectrum
+// stores, the walk) is conflict-free for this lane assignment.  Bounds as in
+// frame_pair_kernel: 8 warps an SM, waiting on their own latencies.
+// ---------------------------------------------------------------------------
+template <int D>
+__global__ void __launch_bounds__(64 * P4Shape::NP, 1) frame_pair4096_kernel(FrontArgs a, int np) {
+  using S = P4Shape;
+  constexpr int N = S::N, M = S::M, TPF = S::TPF, PS = S::PS, threads = 64 * S::NP;
+  griddep_launch();
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int nmel = a.n_mels;
+  const float ref_db = 10.0f * log10f(a.ref);
+  const bool lanes = a.mel_lane_ok != 0;
+  unsigned char *sp = smem;
+  float4 *tw4 = reinterpret_cast<float4 *>(sp);  // as frame_pair_kernel
+  sp += size_t(16) * TPF * 16;
+  float4 *win_s = reinterpret_cast<float4 *>(sp);
+  sp += size_t(N) * 4;
+  // real-split factors: row 2p + j0, column c holds those of c + 32 (4p + j0)
+  // and c + 32 (4p + 2 + j0)
+  float4 *rs_tw = reinterpret_cast<float4 *>(sp);
+  sp += size_t(S::RS) * 16;
+  float4 *wa_s = reinterpret_cast<float4 *>(sp);
+  if (lanes) sp += size_t(16) * 16 * TPF;
+  float2 *wb_s = reinterpret_cast<float2 *>(sp);
+  if (lanes) sp += size_t(16) * 8 * TPF;
+  int4 *lane_s = reinterpret_cast<int4 *>(sp);
+  if (lanes) sp += size_t(16) * TPF;
+  cpx2 *bufs = reinterpret_cast<cpx2 *>(sp);
+  sp += size_t(np) * S::BS * 16;
+  const int words = lanes ? nmel : a.mel_nnz;
+  const bool staged = words <= S::MEL_SMEM_MAX;
+  int *words_s = reinterpret_cast<int *>(sp);
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int fp = warp >> 1;                // this warp's pair
+  const int half = warp & 1;               // 0: even columns, 1: odd columns
+  const int j = half * 32 + lane;          // stage-1 row, walk lane
+  const int j0 = lane & 1;                 // stage-2 half of the column
+  const int col = 2 * (lane >> 1) + half;  // stage-2 column k1
+  const bool c0 = col == 0;
+  const int partner = 2 * (half ? 15 - (lane >> 1) : (16 - (lane >> 1)) & 15) + (1 - j0);
+  const float2 *twq = a.tw_split;  // W_N^t, t < N/4
+
+  for (int i = tid; i < 16 * TPF; i += threads) {
+    const int k = i / TPF, jj = i - k * TPF;
+    const cpx u = root_q(twq, 2 * jj * k, N), w = root_q(twq, 2 * jj * (k + 16), N);
+    tw4[i] = make_float4(u.x, u.y, w.x, w.y);
+  }
+  for (int i = tid; i < 16 * TPF; i += threads) {  // halved: see the header comment
+    const int p = i / TPF, jj = i - p * TPF;
+    const float2 u = __ldg(reinterpret_cast<const float2 *>(a.window) + jj + TPF * (2 * p));
+    const float2 w = __ldg(reinterpret_cast<const float2 *>(a.window) + jj + TPF * (2 * p + 1));
+    win_s[i] = make_float4(0.5f * u.x, 0.5f * u.y, 0.5f * w.x, 0.5f * w.y);
+  }
+  for (int i = tid; i < S::RS; i += threads) {
+    const int row = i / 33, c = min(i - 33 * row, 31), p = row >> 1, jj0 = row & 1;  // (column 32 is padding)
+    const float2 u = split_factors(root_q(twq, c + 32 * (4 * p + jj0), N), p < 4);
+    const float2 w = split_factors(root_q(twq, c + 32 * (4 * p + 2 + jj0), N), p < 4);
+    rs_tw[i] = make_float4(u.x, u.y, w.x, w.y);
+  }
+  bool twice = lanes && stage_walk<TPF>(a, wa_s, wb_s, lane_s, tid, threads);
+  const int *src_words = lanes ? a.mel_band : reinterpret_cast<const int *>(a.mel_pw);
+  if (staged)
+    for (int i = tid; i < words; i += threads) words_s[i] = __ldg(src_words + i);
+  const int *band = staged ? words_s : src_words;
+  twice = __syncthreads_or(twice) != 0;
+  griddep_wait();  // the tables are constant; the clips and their maxima are not
+  if (fp >= np) return;  // a small batch: this warp only helped to stage the tables
+
+  const WarpPairSync sync{fp};
+  cpx2 *fb = bufs + fp * S::BS;
+  f2 *P = reinterpret_cast<f2 *>(fb);
+  cpx2 *parts = reinterpret_cast<cpx2 *>(P + PS * TPF);
+
+  Units<S::UF, S::UT> units(a, fp, np);
+  int vclip = -1;  // the clip vmax belongs to
+  float vmax = -INFINITY;
+  while (units.advance(a)) {  // uniform over the warp pair
+    if (units.clip != vclip) {
+      flush_max(a, vclip, vmax, lane);
+      vclip = units.clip;
+      vmax = -INFINITY;
+    }
+    const ClipDesc &cd = units.cd;
+    const int t = units.first_frame();
+    const bool vb = t + 1 < cd.n_frames;
+    float *dst = a.out + (cd.frame_off + t) * (long long)nmel;
+
+    cpx2 e[16], o[16];
+    load_pair<TPF, D>(a, cd, t, j, win_s, e, o);
+    {  // the samples that the next unit adds, into L1: one line a thread
+      const long long at = (long long)(t + S::UF * np) * a.hop - a.pad + N - (S::UF - 1) * a.hop + j * 32;
+      if (j * 32 < S::UF * a.hop && at >= 0 && at < cd.length)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.signal + cd.sig_off + at));
+    }
+    // ---- stage 1
+    dft16(e);
+    dft16(o);
+    sync();  // the previous unit's reads of the buffer are done
+    finish_stage1<TPF>(e, o, tw4 + j, [&](auto ki, cpx2 y) { fb[j * 33 + decltype(ki)::value] = y; });
+    sync();
+    // ---- stage 2a: 32-point DFT of rows j0 + 2 j1 of column col -> A_j0[q]
+    cpx2 v[32];
+#pragma unroll
+    for (int j1 = 0; j1 < 32; j1++) v[j1] = fb[(j0 + 2 * j1) * 33 + col];
+    dft32(v);
+    // ---- stage 2b: combine the column's two halves; z[i] = Z[col + 32 (2i + j0)],
+    // z[16 + i] = Z[col + 32 (2i + j0 + 32)]
+    cpx2 z[32];
+    static_for<0, 16>([&](auto ii) {
+      constexpr int i = decltype(ii)::value;
+      const cpx2 snd = csel(j0, v[2 * i], v[2 * i + 1]);
+      const cpx2 rcv = {shfl2(snd.x, lane ^ 1), shfl2(snd.y, lane ^ 1)};
+      const cpx2 ev = csel(j0, rcv, v[2 * i]);
+      constexpr float ca = (float)ce_trig(2 * i, 64, 0), sa = -(float)ce_trig(2 * i, 64, 1);
+      constexpr float cb = (float)ce_trig(2 * i + 1, 64, 0), sb = -(float)ce_trig(2 * i + 1, 64, 1);
+      const cpx2 od = cmul(csel(j0, v[2 * i + 1], rcv), {j0 ? cb : ca, j0 ? sb : sa});
+      z[i] = cadd(ev, od);
+      z[16 + i] = csub(ev, od);
+    });
+    sync();  // every column is read: the buffer becomes P
+    // ---- real split: pair i is (Z[k], Z[M - k]), k = col + 32 (2i + j0); the
+    // partner's z[31 - i] holds Z[M - k] (column 0: this thread's own z)
+    {
+      f2 *Pa = P + col + PS * j0;                                       // bin col + 32 s at col + PS s
+      f2 *Pb = P + (PS * (TPF - 1) + 32 - col - PS * j0) + (c0 ? 1 : 0);  // bin M - col - 32 s
+      float4 rsp;
+      cpx2 prev = z[0];
+      static_for<0, 16>([&](auto ii) {
+        constexpr int i = decltype(ii)::value;
+        const cpx2 up = z[31 - i];
+        const cpx2 rcv = {shfl2(up.x, partner), shfl2(up.y, partner)};
+        const cpx2 zb = csel(c0, csel(j0, up, prev), rcv);
+        prev = up;
+        if constexpr (i % 2 == 0) rsp = rs_tw[(i + j0) * 33 + col];  // row 2 (i / 2) + j0
+        f2 p, q;
+        split_pair<(i < 8)>(z[i], zb, i % 2 == 0 ? rsp.x : rsp.z, i % 2 == 0 ? rsp.y : rsp.w, p, q);
+        Pa[2 * PS * i] = p;
+        if constexpr (i == 0) Pb[(c0 && !j0) ? -1 : 0] = q;  // column 0, s = 0: the Nyquist bin
+        else Pb[-2 * PS * i] = q;
+      });
+      if (c0 && !j0) P[M / 2 + TPF / 2] = mul2(dup2(4.0f), fma2(prev.x, prev.x, mul2(prev.y, prev.y)));
+    }
+    sync();  // P complete
 
     // ---- log-mel rows of both frames + running clip max
-    if (lanes) {
-      // Lane l sums its 32 bins (the last lane also the Nyquist bin) into
-      // (R, F) = (rising, falling weight) times P and stores the sums in the
-      // next part slot at every segment end.  Bins go in pairs: the second
-      // bin of a pair has its weights in one of two sets, zero in the other,
-      // (wa.z, wa.w) for the segment that the first bin belongs to and wb for
-      // a segment that it starts, so one predicated store and restart serve
-      // a pair wherever in it the segment ends.  Pairs that end two segments
-      // (bands of a single bin) take the second end in a branch of their own.
-      const int4 li = lane_s[l];
-      const unsigned fl = (unsigned)li.x;
-      const uint32_t part0 = smem_u32(parts);
-      uint32_t at = part0 + (unsigned)li.y;  // the next part's slot
-      const float4 *pl = reinterpret_cast<const float4 *>(P + PS * l);
-      const float4 *wa = wa_s + l;
-      const float2 *wb = wb_s + l;
-      const f2 zero = dup2(0.0f);
-      f2 R = zero, Fs = zero;
-      // the frames' non-finite check: the largest bit pattern of a power (a
-      // power is never negative; NaN and inf lie at or above inf's pattern)
-      unsigned mxa = 0u, mxb = 0u;
-      static_for<0, 16>([&](auto gi) {
-        constexpr int g = decltype(gi)::value;
-        const float4 pq = pl[g], u = wa[g * TPF];
-        const float2 w = wb[g * TPF];
-        mxa = max(max(mxa, __float_as_uint(pq.x)), __float_as_uint(pq.z));
-        mxb = max(max(mxb, __float_as_uint(pq.y)), __float_as_uint(pq.w));
-        const f2 p0 = pk2(pq.x, pq.y), p1 = pk2(pq.z, pq.w);
-        R = fma2(p0, dup2(u.x), R);
-        Fs = fma2(p0, dup2(u.y), Fs);
-        R = fma2(p1, dup2(u.z), R);
-        Fs = fma2(p1, dup2(u.w), Fs);
-        walk_end<g>(p1, w.x, w.y, fl, R, Fs, at);
-        if (twice && (fl & (0x10000u << g))) {
-          walk_store(at, R, Fs);
-          at += 16;
-          R = zero;
-          Fs = zero;
-        }
-      });
-      if (l == TPF - 1) {
-        if (__ldg(a.mel_lane + l).x < 0) {  // bin 31 ends a segment
-          walk_store(at, R, Fs);
-          at += 16;
-          R = zero;
-          Fs = zero;
-        }
-        const float4 pq = pl[16];
-        const float2 w = __ldg(a.mel_lw + 32 * TPF + l);
-        mxa = max(mxa, __float_as_uint(pq.x));
-        mxb = max(mxb, __float_as_uint(pq.y));
-        R = fma2(pk2(pq.x, pq.y), dup2(w.x), R);
-        Fs = fma2(pk2(pq.x, pq.y), dup2(w.y), Fs);
-      }
-      walk_store(at, R, Fs);
-      if (l == 0) parts[li.w] = {zero, zero};  // the empty segments' slot
-      const unsigned ba = __ballot_sync(FULL, mxa >= 0x7f800000u), bb = __ballot_sync(FULL, mxb >= 0x7f800000u);
-      // added to a frame's band sums: NaN where a bin of it is not finite
-      const f2 nan2 = pk2((ba & gmask) ? __int_as_float(0x7fc00000) : 0.0f, (bb & gmask) ? __int_as_float(0x7fc00000) : 0.0f);
-      __syncwarp();
-      // a lane whose last part heads a segment adds the parts of the lanes the
-      // segment runs into
-      if (li.z) {
-        cpx2 *h = parts + ((at - part0) >> 4);
-        cpx2 hv = *h;
-        for (int j = 1; j <= li.z; j++) hv = cadd(hv, h[j]);
-        *h = hv;
-      }
-      __syncwarp();
-      // band m is the head of segment m (rising) plus the head of segment
-      // m + 1 (falling); four bands at a time, so that their reads overlap.
-      // The lane tables hold finite weights only: no band is NaN by itself.
-      const char *pb = reinterpret_cast<const char *>(parts);
-      for (int m0 = l; m0 < nmel; m0 += 4 * TPF) {
-        int bw[4];
-        f2 acc[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) bw[i] = m0 + i * TPF < nmel ? band[m0 + i * TPF] : 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-          acc[i] = add2(*reinterpret_cast<const f2 *>(pb + 16 * (bw[i] & 4095)),
-                        *reinterpret_cast<const f2 *>(pb + 8 + 16 * ((bw[i] >> 12) & 4095)));
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const int m = m0 + i * TPF;
-          float xa, xb;
-          un2(add2(acc[i], nan2), xa, xb);
-          const float da = fmaf(k10Log10of2, __log2f(fmaxf(xa, a.amin)), -ref_db);
-          const float db = fmaf(k10Log10of2, __log2f(fmaxf(xb, a.amin)), -ref_db);
-          if (va && m < nmel) {
-            dst[m] = da;
-            vmax = fmaxf(vmax, da);
-          }
-          if (vb && m < nmel) {
-            dst[nmel + m] = db;
-            vmax = fmaxf(vmax, db);
-          }
-        }
-      }
-    } else {
-      unsigned mxa = 0u, mxb = 0u;  // the non-finite check: this lane's share of the bins
-      for (int k = l; k <= M; k += TPF) {
-        float pa, pb;
-        un2(P[pair_bin<TPF>(k)], pa, pb);
-        mxa = max(mxa, __float_as_uint(pa));
-        mxb = max(mxb, __float_as_uint(pb));
-      }
-      const bool bada = (__ballot_sync(FULL, mxa >= 0x7f800000u) & gmask) != 0;
-      const bool badb = (__ballot_sync(FULL, mxb >= 0x7f800000u) & gmask) != 0;
-      for (int m = l; m < nmel; m += TPF) {
-        const int4 info = __ldg(a.mel_info + m);
-        const float *wr = melw + info.z;
-        f2 acc = dup2(0.0f);
-        for (int q = 0; q < info.y; q++) acc = fma2(P[pair_bin<TPF>(info.x + q)], dup2(wr[q]), acc);
-        float xa, xb;
-        un2(acc, xa, xb);
-        if (info.w || bada) xa = __int_as_float(0x7fc00000);
-        if (info.w || badb) xb = __int_as_float(0x7fc00000);
-        if (va) {
-          const float val = db10_frame(xa, a.amin, ref_db);
-          dst[m] = val;
-          vmax = fmaxf(vmax, val);
-        }
-        if (vb) {
-          const float val = db10_frame(xb, a.amin, ref_db);
-          dst[nmel + m] = val;
-          vmax = fmaxf(vmax, val);
-        }
-      }
-    }
+    if (lanes) walk_bands<TPF>(a, sync, P, parts, j, {wa_s, wb_s, lane_s, band, twice}, ref_db, dst, true, vb, vmax);
+    else row_bands<TPF>(a, sync, P, j, reinterpret_cast<const float *>(band), ref_db, dst, true, vb, vmax);
   }
-  float m = vmax;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
-  if (lane == 0 && vclip >= 0 && m > -INFINITY) atomicMax(a.clip_max + vclip, enc_f(m));
+  flush_max(a, vclip, vmax, lane);
 }
 
 static int sm_count_cached() {
@@ -660,31 +923,50 @@ static int sm_count_cached() {
   return n;
 }
 
-template <int LOG2N, int D>
-static cudaError_t launch_pair_d(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched) {
-  using S = PShape<LOG2N>;
+// One CTA per SM, and as few of its warps (or warp pairs) at work as finish in
+// the same number of rounds: a small batch spreads over all SMs (all warps
+// stage the tables: a 3 s clip, one unit an SM, waits for nothing else).
+// smem_of(w): shared memory with w workers.
+template <typename K, typename Smem>
+static cudaError_t launch_units(K kern, const FrontArgs &a, int per_tile, int workers, int threads, Smem smem_of,
+                                int grid_limit, cudaStream_t s, int *launched) {
   int per_sm = 1, sms = sm_count_cached();
   if (grid_limit > 0 && sms > grid_limit) sms = grid_limit;
-  // One CTA per SM, and as few of its warps at work as finish in the same
-  // number of rounds: a small batch spreads over all SMs (all warps stage the
-  // tables: a 3 s clip, one unit an SM, waits for nothing else).
-  const long long units = (long long)a.total_tiles * S::UT;
-  const long long rounds = (units + (long long)sms * S::NW - 1) / ((long long)sms * S::NW);
-  const int nw = (int)((units + sms * rounds - 1) / (sms * rounds));
-  const int words = a.mel_lane_ok ? a.n_mels : a.mel_nnz;
-  const size_t smem = pair_fixed_smem<LOG2N>() + (a.mel_lane_ok ? (16 * 24 + 16) * (size_t)S::TPF : 0) +
-                      nw * pair_warp_smem<LOG2N>() + (words <= S::MEL_SMEM_MAX ? align16(4 * (size_t)words) : 0);
-  auto kern = frame_pair_kernel<LOG2N, D>;
-  cudaError_t e = persistent_geometry(reinterpret_cast<const void *>(kern), 32 * S::NW, smem, &per_sm, &sms);
+  const long long units = (long long)a.total_tiles * per_tile;
+  const long long rounds = (units + (long long)sms * workers - 1) / ((long long)sms * workers);
+  const int w = (int)((units + sms * rounds - 1) / (sms * rounds));
+  const size_t smem = smem_of(w);
+  int all = 0;
+  cudaError_t e = persistent_geometry(reinterpret_cast<const void *>(kern), threads, smem, &per_sm, &all);
   if (e != cudaSuccess) return e;
-  long long grid = sms;
-  if (grid_limit > 0 && grid > grid_limit) grid = grid_limit;
-  if (grid > units) grid = units;
+  const long long grid = units < sms ? units : sms;
   if (grid < 1) return cudaSuccess;
-  e = launch_after(kern, (unsigned)grid, 32 * S::NW, smem, s, a, nw);
+  e = launch_after(kern, (unsigned)grid, threads, smem, s, a, w);
   if (e != cudaSuccess) return e;
   if (launched) *launched = (int)grid;
   return cudaGetLastError();
+}
+
+template <int LOG2N, int D>
+static cudaError_t launch_pair_d(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched) {
+  using S = PShape<LOG2N>;
+  const int words = a.mel_lane_ok ? a.n_mels : a.mel_nnz;
+  auto smem_of = [&](int w) {
+    return pair_fixed_smem<LOG2N>() + (a.mel_lane_ok ? (16 * 24 + 16) * (size_t)S::TPF : 0) +
+           w * pair_warp_smem<LOG2N>() + (words <= S::MEL_SMEM_MAX ? align16(4 * (size_t)words) : 0);
+  };
+  return launch_units(frame_pair_kernel<LOG2N, D>, a, S::UT, S::NW, 32 * S::NW, smem_of, grid_limit, s, launched);
+}
+
+template <int D>
+static cudaError_t launch_pair4096_d(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched) {
+  using S = P4Shape;
+  const int words = a.mel_lane_ok ? a.n_mels : a.mel_nnz;
+  auto smem_of = [&](int w) {
+    return S::fixed + (a.mel_lane_ok ? S::walk : 0) + w * size_t(S::BS) * 16 +
+           (words <= S::MEL_SMEM_MAX ? align16(4 * (size_t)words) : 0);
+  };
+  return launch_units(frame_pair4096_kernel<D>, a, S::UT, S::NP, 64 * S::NP, smem_of, grid_limit, s, launched);
 }
 
 template <int LOG2N>
@@ -700,6 +982,9 @@ cudaError_t launch_frontend_pair(int log2n, const FrontArgs &a, int grid_limit, 
     case 9: return launch_pair<9>(a, grid_limit, s, launched);
     case 10: return launch_pair<10>(a, grid_limit, s, launched);
     case 11: return launch_pair<11>(a, grid_limit, s, launched);
+    case 12:
+      if (a.hop == 1024 && a.even_starts) return launch_pair4096_d<8>(a, grid_limit, s, launched);
+      return launch_pair4096_d<0>(a, grid_limit, s, launched);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -153,8 +153,7 @@ cudaError_t launch_stack_memory(const float *x, float *y, int n_features, int n_
 int frames_per_tile(int log2n, int variant);
 // Number of launch variants the autotuner may choose from (1 = not tunable).
 int frame_variants(int log2n, int mode, int power_is_2);
-// Launch variant 3 (MODE_MELDB): the frame-pair kernel for n_fft 256..2048, the
-// warp-pair kernel for 4096.
+// Launch variant 3 (MODE_MELDB, n_fft 256..4096): the frame-pair kernels.
 constexpr int kWarpVariant = 3;
 // Launch variant of the tensor-core frame kernel (n_fft 2048, MFCC path):
 // both 32-point DFT stages as fp16x3 tcgen05 GEMMs, 16 frames per tile.
@@ -180,8 +179,6 @@ inline int mel_lane_max_slots(int tpf) {
 }
 cudaError_t launch_frontend_tc(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched);
 cudaError_t launch_frontend_pair(int log2n, const FrontArgs &a, int grid_limit, cudaStream_t s,
-                                 int *launched);
-cudaError_t launch_frontend_warp(int log2n, const FrontArgs &a, int grid_limit, cudaStream_t s,
                                  int *launched);
 // Stockham twiddle table length (entries) for log2(n_fft) >= 5.
 int stage_twiddle_count(int log2n);

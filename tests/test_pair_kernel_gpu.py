@@ -1,4 +1,4 @@
-"""The frame-pair kernel (launch variant 3, n_fft 256..2048): two frames at a
+"""The frame-pair kernels (launch variant 3, n_fft 256..4096): two frames at a
 time, so the cases are the places where a pair can go wrong: one, two and
 three frames, odd frame counts, clips shorter than a frame, edge pairs under
 both paddings, the shared gather of hop n_fft/4 beside any other hop (odd
@@ -53,6 +53,7 @@ def _rows(variant, clips, n_mels, **params):
     (1024, 256, 64), (1024, 441, 128), (1024, 256, 260),
     (512, 128, 40), (512, 160, 80), (512, 128, 200),
     (256, 64, 40), (256, 85, 26), (256, 64, 120),
+    (4096, 1024, 128), (4096, 441, 64), (4096, 2048, 40), (4096, 1024, 900), (4096, 1024, 1100),
 ])
 def test_pair_kernel_vs_cta_tile_kernel_and_oracle(n_fft, hop, n_mels, pad):
     sr = 22050
@@ -73,7 +74,7 @@ def test_pair_kernel_vs_cta_tile_kernel_and_oracle(n_fft, hop, n_mels, pad):
                 assert O.mfcc_rel_error(c, exp) < MFCC_TOL, (len(y), center)
 
 
-@pytest.mark.parametrize("n_fft,n_mels", [(2048, 128), (2048, 1100), (512, 40)])
+@pytest.mark.parametrize("n_fft,n_mels", [(2048, 128), (2048, 1100), (512, 40), (4096, 128), (4096, 1100)])
 def test_pair_kernel_flags_only_the_frame_with_a_non_finite_sample(n_fft, n_mels):
     """A NaN reaches the frames that cover it and no other: the partner frame
     of a pair and its neighbours keep their values bit for bit."""
