@@ -3,12 +3,14 @@
 
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 
 #include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 namespace mm {
@@ -468,12 +470,31 @@ size_t pool_class(size_t bytes) {
 }
 }  // namespace
 
+namespace {
+// Blocks are private anonymous memory, page-locked in place: after a fork the
+// child has copies of them as of any other memory (cudaHostAlloc's blocks were
+// shared, and a child's writes appeared in its parent's arrays).
+void *block_new(size_t bytes) {
+  void *p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_POPULATE, -1, 0);
+  if (p == MAP_FAILED) return nullptr;
+  if (cudaHostRegister(p, bytes, cudaHostRegisterPortable) == cudaSuccess) return p;
+  cudaGetLastError();
+  munmap(p, bytes);
+  return nullptr;
+}
+void block_delete(void *p, size_t bytes) {
+  // memory that could not be unlocked (a driver already shut down) stays mapped
+  if (cudaHostUnregister(p) == cudaSuccess) munmap(p, bytes);
+  else cudaGetLastError();
+}
+}  // namespace
+
 float *result_alloc(size_t bytes, bool pooled, bool *pinned) {
   *pinned = false;
   if (pooled && bytes >= kPoolMin && bytes <= kPoolCap / 2) {
     ResultPool &rp = result_pool();
     const size_t cls = pool_class(bytes);
-    std::vector<void *> drop;
+    std::vector<std::pair<size_t, void *>> drop;
     bool fits = false;
     {
       std::lock_guard<std::mutex> lock(rp.mu);
@@ -489,7 +510,7 @@ float *result_alloc(size_t bytes, bool pooled, bool *pinned) {
       if (rp.total + cls > kPoolCap && ++rp.refused >= 16) {  // idle blocks of sizes no longer asked for
         for (auto &b : rp.idle) {
           rp.total -= b.first;
-          drop.push_back(b.second);
+          drop.push_back(b);
         }
         rp.idle.clear();
         rp.refused = 0;
@@ -499,17 +520,15 @@ float *result_alloc(size_t bytes, bool pooled, bool *pinned) {
         fits = true;
       }
     }
-    for (void *p : drop) cudaFreeHost(p);
+    for (auto &b : drop) block_delete(b.second, b.first);
     if (fits) {
-      void *p = nullptr;
-      const cudaError_t e = cudaHostAlloc(&p, cls, cudaHostAllocPortable);
+      void *p = block_new(cls);
       std::lock_guard<std::mutex> lock(rp.mu);
-      if (e == cudaSuccess) {
+      if (p) {
         rp.live[p] = cls;
         *pinned = true;
         return static_cast<float *>(p);
       }
-      cudaGetLastError();
       rp.total -= cls;
     }
   }

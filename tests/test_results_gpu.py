@@ -5,6 +5,7 @@ threads, and for views and in-place changes; results released through the C
 ABI go back the same way."""
 
 import gc
+import os
 import threading
 
 import numpy as np
@@ -81,3 +82,22 @@ def test_c_abi_contexts_of_both_kinds_give_the_same_values():
     a = take_buffer(out)
     assert out.data == ffi.NULL
     np.testing.assert_array_equal(a.ravel(), got[0])
+
+
+def test_a_forked_child_has_its_own_copy():
+    """As with any array: a child reads what was there, its writes stay with it,
+    and the block goes on receiving results in the parent."""
+    y = _clip(11)
+    a = M.stft(y)
+    want = a.copy()
+    pid = os.fork()
+    if pid == 0:  # no CUDA here
+        same = np.array_equal(a, want)
+        a[:] = -1.0
+        os._exit(0 if same else 3)
+    assert os.waitpid(pid, 0)[1] == 0
+    np.testing.assert_array_equal(a, want)
+    del a
+    gc.collect()
+    for _ in range(3):
+        np.testing.assert_array_equal(M.stft(y), want)
