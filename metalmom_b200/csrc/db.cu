@@ -12,13 +12,20 @@
 //   every block of the second kernel reduces for itself; no slots to reset, no
 //   atomics.  The second kernel walks x from its end, where the first one left
 //   it in L2.
-// Bound by HBM: 42.3 M values (169 MB, more than L2) with ref = max(x): see the
-// figures at launch_db.
+//
+// The logarithm was what the second pass spent its time on (42.3 M values, 169
+// MB, ref = max(x): 86 us where its 338 MB take 52), an IEEE division and a
+// log10f a value.  Values whose quotient is surely a normal float32 now go two
+// at a time in packed arithmetic (db_pair): the call 120 -> 106 us (the first
+// pass takes 28 of it), its error against float64 3.7e-8 -> 2.0e-8.  Measured
+// and left out: six resident blocks an SM instead of five (107 us), streaming
+// stores (107 us).
 //
 // amin <= 0 (or NaN) keeps the pass-by-pass form: a logarithm of a negative
 // number is NaN and the maximum must skip it.
 #include <math.h>
 
+#include "f32x2.cuh"
 #include "frame_common.cuh"
 #include "kernels.h"
 
@@ -49,12 +56,79 @@ __device__ __forceinline__ void block_max(float &vmax, bool &nan) {
   vmax = v;
 }
 
-// Reference value and floor from max(x) (NaNs skipped) and "x holds a NaN".
-__device__ __forceinline__ void db_levels(float xmax, bool nan, bool ref_max, float mult, float amin, float top_db,
-                                          float &ref, float &thr) {
+// What a launch's values have in common.
+struct Levels {
+  float mult, amin, ref, thr;  // thr: the floor (-inf: none)
+  bool packed;                 // db_pair applies to values up to kPairHigh
+  bool all;                    // ... and no value is larger
+  float inv, twice;            // its 1 / ref, and mult / 10
+};
+// Range of db_pair: which form a value takes depends on it, amin and ref
+// alone, so that every route gives it the same result.
+constexpr float kPairLow = 8.67361737988403547e-19f, kPairHigh = 1.152921504606846976e18f;  // 2^-60, 2^60
+
+// mult log10(x / ref) of two values where x, ref and so the quotient are well
+// inside the normal range.
+// - Quotient: with inv the correctly rounded 1 / ref, one residual step from
+//   x inv gives the correctly rounded x / ref (Markstein, IBM J. Res. Dev. 34,
+//   1990), the value that db_value takes the logarithm of.
+// - Logarithm: x / ref = 2^e (1 + f) with 1 + f in [sqrt(1/2), sqrt(2)), and
+//   10 log10(1 + f) = c f + f^2 Q(f), Q the weighted least-squares polynomial of degree 9
+//   at Chebyshev points (its error: 1e-9 of the result).  c and 10 log10(2) are carried in two
+//   floats, so the result is off by little more than its last rounding.
+__device__ __forceinline__ f2 db_pair(f2 x, const Levels &lv) {
+  const f2 inv = dup2(lv.inv);
+  const f2 q0 = mul2(x, inv);
+  const f2 q = fma2(fma2(neg2(q0), dup2(lv.ref), x), inv, q0);
+  float qa, qb;
+  un2(q, qa, qb);
+  const int ia = __float_as_int(qa), ib = __float_as_int(qb);
+  constexpr int kSqrtHalf = 0x3f3504f3, kBias = 0x4b400000;  // kBias: 1.5 2^23, to which e is added as an integer
+  const int ta = ia - kSqrtHalf, tb = ib - kSqrtHalf;
+  const f2 m = pk2(__int_as_float(ia - (ta & 0xff800000)), __int_as_float(ib - (tb & 0xff800000)));
+  const f2 e = sub2(pk2(__int_as_float((ta >> 23) + kBias), __int_as_float((tb >> 23) + kBias)), dup2(12582912.0f));
+  const f2 f = sub2(m, dup2(1.0f));
+  constexpr float kQ[10] = {-2.1714723110198975f, 1.4476473331451416f,  -1.0857372283935547f, 0.8686825633049011f,
+                            -0.7238692045211792f, 0.6175169944763184f,  -0.5388593673706055f, 0.5165238976478577f,
+                            -0.5068863034248352f, 0.2925231456756592f};
+  f2 g = dup2(kQ[9]);
+#pragma unroll
+  for (int i = 8; i >= 0; i--) g = fma2(g, f, dup2(kQ[i]));
+  g = fma2(g, f, dup2(1.9699272335452558e-07f));  // 10 / ln 10 = 4.342944622039795 + this
+  f2 y = fma2(f, dup2(4.342944622039795f), mul2(f, g));
+  y = fma2(e, dup2(3.560404593372368e-08f), y);  // 10 log10(2) = 3.0102999210357666 + this
+  y = fma2(e, dup2(3.0102999210357666f), y);
+  return mul2(y, dup2(lv.twice));
+}
+
+__device__ __forceinline__ Levels levels(float mult, float amin, float ref) {
+  Levels lv{mult, amin, ref, -INFINITY, false, false, 0.0f, 1.0f};
+  lv.packed = amin >= kPairLow && amin <= kPairHigh && ref >= kPairLow && ref <= kPairHigh &&  // false for NaN
+              (mult == 10.0f || mult == 20.0f);
+  if (lv.packed) lv.inv = 1.0f / ref;
+  if (mult == 20.0f) lv.twice = 2.0f;
+  return lv;
+}
+// dB of two values
+__device__ __forceinline__ void db_two(float &a, float &b, const Levels &lv) {
+  const float xa = vthr(a, lv.amin), xb = vthr(b, lv.amin);
+  if (lv.packed && (lv.all || fmaxf(xa, xb) <= kPairHigh)) {
+    un2(db_pair(pk2(xa, xb), lv), a, b);
+  } else {
+    a = lv.packed && xa <= kPairHigh ? lo2(db_pair(dup2(xa), lv)) : db_value(a, lv.mult, lv.amin, lv.ref);
+    b = lv.packed && xb <= kPairHigh ? lo2(db_pair(dup2(xb), lv)) : db_value(b, lv.mult, lv.amin, lv.ref);
+  }
+}
+// The same with what follows from max(x) (NaNs skipped) and "x holds a NaN".
+__device__ __forceinline__ Levels levels_of_max(float xmax, bool nan, float ref, bool ref_max, float mult, float amin,
+                                                float top_db) {
   if (ref_max) ref = nan ? __int_as_float(0x7fc00000) : xmax;
-  const float top = db_value(xmax, mult, amin, ref);
-  thr = top_db > 0.0f ? (isnan(top) ? -INFINITY : top) - top_db : -INFINITY;
+  Levels lv = levels(mult, amin, ref);
+  lv.all = lv.packed && xmax <= kPairHigh;
+  float top = xmax, unused = xmax;
+  db_two(top, unused, lv);
+  if (top_db > 0.0f) lv.thr = (isnan(top) ? -INFINITY : top) - top_db;
+  return lv;
 }
 
 // 4 values in, 4 out; the tail and unaligned buffers one by one.
@@ -84,6 +158,15 @@ __device__ __forceinline__ void store_quad(float *y, long long i, long long n, b
       if (i + k < n) y[i + k] = q.v[k];
   }
 }
+// dB values of a quad with their floor.
+__device__ __forceinline__ void db_quad(Quad &q, const Levels &lv, bool floor_on) {
+  db_two(q.v[0], q.v[1], lv);
+  db_two(q.v[2], q.v[3], lv);
+  if (floor_on) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) q.v[k] = vthr(q.v[k], lv.thr);
+  }
+}
 __device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_cast<size_t>(p) & 15) == 0; }
 
 // x and y may be the same buffer: a thread reads what it writes, before it.
@@ -103,18 +186,12 @@ __global__ void __launch_bounds__(kDbSmallThreads) db_small_kernel(const float *
     }
   }
   block_max<kDbSmallThreads>(vmax, nan);
-  float thr;
-  db_levels(vmax, nan, ref_max, mult, amin, top_db, ref, thr);
-  const bool floor_on = top_db > 0.0f;
+  const Levels lv = levels_of_max(vmax, nan, ref, ref_max, mult, amin, top_db);
 #pragma unroll
   for (int u = 0; u < kDbSmallPer; u++) {
     const long long i = 4LL * (threadIdx.x + u * kDbSmallThreads);
     if (i >= n) break;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float v = db_value(q[u].v[k], mult, amin, ref);
-      q[u].v[k] = floor_on ? vthr(v, thr) : v;
-    }
+    db_quad(q[u], lv, top_db > 0.0f);
     store_quad(y, i, n, vy, q[u]);
   }
 }
@@ -154,7 +231,7 @@ __global__ void __launch_bounds__(kDbThreads) db_max_kernel(const float *x, long
 __global__ void __launch_bounds__(kDbThreads) db_apply_kernel(const float *x, float *y, long long n, float mult,
                                                               float amin, float ref, bool ref_max, float top_db,
                                                               const float2 *part, int n_part) {
-  float thr = -INFINITY;
+  Levels lv = levels(mult, amin, ref);
   if (n_part > 0) {
     float vmax = -INFINITY;
     bool nan = false;
@@ -164,18 +241,24 @@ __global__ void __launch_bounds__(kDbThreads) db_apply_kernel(const float *x, fl
       nan |= p.y != 0.0f;
     }
     block_max<kDbThreads>(vmax, nan);
-    db_levels(vmax, nan, ref_max, mult, amin, top_db, ref, thr);
+    lv = levels_of_max(vmax, nan, ref, ref_max, mult, amin, top_db);
   }
   const bool floor_on = top_db > 0.0f, vx = aligned16(x), vy = aligned16(y);
   const long long quads = (n + 3) / 4, step = (long long)kDbThreads * gridDim.x;
-  for (long long j = blockIdx.x * (long long)kDbThreads + threadIdx.x; j < quads; j += step) {
-    const long long i = 4 * (quads - 1 - j);  // from the end: what db_max_kernel read last
+  // from the end, which db_max_kernel read last; two loads in flight
+  long long j = blockIdx.x * (long long)kDbThreads + threadIdx.x;
+  for (; j + step < quads; j += 2 * step) {
+    const long long i = 4 * (quads - 1 - j), i2 = i - 4 * step;
+    Quad q = load_quad(x, i, n, vx, 0.0f), q2 = load_quad(x, i2, n, vx, 0.0f);
+    db_quad(q, lv, floor_on);
+    store_quad(y, i, n, vy, q);
+    db_quad(q2, lv, floor_on);
+    store_quad(y, i2, n, vy, q2);
+  }
+  if (j < quads) {
+    const long long i = 4 * (quads - 1 - j);
     Quad q = load_quad(x, i, n, vx, 0.0f);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const float v = db_value(q.v[k], mult, amin, ref);
-      q.v[k] = floor_on ? vthr(v, thr) : v;
-    }
+    db_quad(q, lv, floor_on);
     store_quad(y, i, n, vy, q);
   }
 }

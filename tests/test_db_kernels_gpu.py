@@ -77,3 +77,24 @@ def test_db_device_special_values(n):
     x[1] = np.nan
     got = M.power_to_db_device(torch.from_numpy(x).cuda(), ref=np.max, top_db=None).cpu().numpy()
     assert np.isnan(got).all()
+
+
+@pytest.mark.parametrize("n", [7, 32768, 100003])
+@pytest.mark.parametrize("scale", [2.0 ** -58, 1e-9, 1.0, 2.0 ** 40, 2.0 ** 59, 2.0 ** 61, 1e38])
+def test_db_device_accuracy_by_magnitude(n, scale):
+    """Both forms of the logarithm (values inside [2^-60, 2^60] and beyond) to a
+    few roundings.  Per 10 dB of `mult`: the quotient's 2^-24 is 2.6e-7 dB, the
+    logarithm of the mantissa (at most 1.51 dB) takes three roundings of 2^-24,
+    2.7e-7 dB (log10f: 2 ulp of y), and the sums and product two of y."""
+    import torch
+    rng = np.random.default_rng(n)
+    x = (scale * np.exp2(rng.uniform(-1.0, 1.0, n))).astype(np.float32)
+    x[::3] = (scale * (1.0 + np.float64(2.0 ** -23) * rng.integers(-40, 40, len(x[::3])))).astype(np.float32)
+    d = torch.from_numpy(x).cuda()
+    for fn, mult in ((M.power_to_db_device, 10.0), (M.amplitude_to_db_device, 20.0)):
+        for amin in (1e-30, float(np.float32(scale))):
+            for ref in (1.0, np.max, float(np.float32(scale * 0.7))):
+                r = float(max(x.max(), np.float32(amin))) if ref is np.max else ref
+                y = fn(d, ref=ref, amin=amin, top_db=100.0).cpu().numpy().astype(np.float64)
+                e = _expected(x, mult, amin, np.float64(r), 100.0)
+                assert (np.abs(y - e) <= 1e-6 * mult / 10 + 2.0 ** -21 * np.abs(e)).all()
