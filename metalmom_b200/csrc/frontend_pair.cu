@@ -40,7 +40,7 @@
 // the kernel now waits on its own latencies (issue 44 %, shared-memory pipe
 // 67 %).  256 clips of 30 s at n_fft 2048, hop 512, 128 bands: 0.90 -> 0.77 ms
 // (whole step 0.954 -> 0.833); 512 clips of 10 s at n_fft 512, hop 160, 80
-// bands, whole step: 0.62 (CTA-tile kernel) -> 0.42.  64 clips of 30 s at 44.1 kHz,
+// bands, whole step: 0.62 (CTA-tile kernel) -> 0.39.  64 clips of 30 s at 44.1 kHz,
 // n_fft 4096, hop 1024: 0.571 -> 0.511 (one frame per warp pair, 16 warps, before).
 // Measured and left out (128 clips, whole step, against 0.426 ms): 12 warps of
 // 168 registers 0.443; the next pair's samples loaded into registers before
@@ -969,10 +969,18 @@ static cudaError_t launch_pair4096_d(const FrontArgs &a, int grid_limit, cudaStr
   return launch_units(frame_pair4096_kernel<D>, a, S::UT, S::NP, 64 * S::NP, smem_of, grid_limit, s, launched);
 }
 
+// Shared gathers exist for the usual hops, each against D = 0 on 64 clips of
+// 30 s (whole step): n_fft/2 at n_fft 256 195 -> 181 us, 512 147 -> 139, 1024
+// 134 -> 135 (one clip: 17.5 -> 16.6), 2048 125 -> 121; 10 ms of 32 ms at n_fft
+// 256 304 -> 274, 512 225 -> 209, 1024 198 -> 197; 512 utterances of 10 s at
+// n_fft 512 420 -> 394.
 template <int LOG2N>
 static cudaError_t launch_pair(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched) {
-  constexpr int step = 2 * PShape<LOG2N>::TPF;  // samples per register step
-  if (a.hop == 8 * step && a.even_starts) return launch_pair_d<LOG2N, 8>(a, grid_limit, s, launched);    // n_fft / 4
+  constexpr int step = 2 * PShape<LOG2N>::TPF;  // samples per register step, n_fft / 32
+  if (a.even_starts && a.hop == 8 * step) return launch_pair_d<LOG2N, 8>(a, grid_limit, s, launched);    // n_fft / 4
+  if (a.even_starts && a.hop == 16 * step) return launch_pair_d<LOG2N, 16>(a, grid_limit, s, launched);  // n_fft / 2
+  if constexpr (LOG2N <= 10)  // 10 ms of a 32 ms frame: speech at 8, 16 and 32 kHz
+    if (a.even_starts && a.hop == 10 * step) return launch_pair_d<LOG2N, 10>(a, grid_limit, s, launched);
   return launch_pair_d<LOG2N, 0>(a, grid_limit, s, launched);
 }
 

@@ -53,6 +53,7 @@ def _rows(variant, clips, n_mels, **params):
     (1024, 256, 64), (1024, 441, 128), (1024, 256, 260),
     (512, 128, 40), (512, 160, 80), (512, 128, 200),
     (256, 64, 40), (256, 85, 26), (256, 64, 120),
+    (1024, 320, 64), (1024, 512, 128), (512, 256, 80), (256, 80, 40), (256, 128, 26),
     (4096, 1024, 128), (4096, 441, 64), (4096, 2048, 40), (4096, 1024, 900), (4096, 1024, 1100),
 ])
 def test_pair_kernel_vs_cta_tile_kernel_and_oracle(n_fft, hop, n_mels, pad):
