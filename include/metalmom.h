@@ -68,6 +68,12 @@ MM_API mm_context mm_init(void);
  * Release them with mm_buffer_free and nothing else. */
 MM_API mm_context mm_init_pooled(void);
 
+/* Additive: as mm_init, but a call on this context whose result has exactly
+ * `count` floats writes it to dst, which stays the caller's memory: MMBuffer.data
+ * is then dst and is not given to mm_buffer_free.  Results of any other size
+ * are malloc'd as usual.  NULL when dst is NULL or count is not positive. */
+MM_API mm_context mm_init_into(float* dst, int64_t count);
+
 /* Replaces Bridge.swift:33 (mm_destroy); destroying twice is a no-op. */
 MM_API void mm_destroy(mm_context ctx);
 

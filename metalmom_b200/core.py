@@ -2,7 +2,7 @@
 
 import numpy as np
 
-from ._bridge import bridge_call, float_ptr, stft_params
+from ._bridge import bridge_call, float_ptr, frame_shape, sample_shape, stft_params
 from ._native import lib
 
 SR_UNUSED = 22050  # the bridge's STFT entry points take a sample rate they do not use
@@ -21,7 +21,8 @@ def stft(y, n_fft=2048, hop_length=None, win_length=None, center=True):
     """
     y, ptr = float_ptr(y)
     hop, win = _defaults(n_fft, hop_length, win_length)
-    return bridge_call("mm_stft", lib.mm_stft, ptr, len(y), SR_UNUSED, stft_params(n_fft, hop, win, center))
+    return bridge_call("mm_stft", lib.mm_stft, ptr, len(y), SR_UNUSED, stft_params(n_fft, hop, win, center),
+                       shape=frame_shape(n_fft // 2 + 1, len(y), n_fft, hop, center))
 
 
 def stft_complex(y, n_fft=2048, hop_length=None, win_length=None, center=True):
@@ -35,7 +36,8 @@ def stft_complex(y, n_fft=2048, hop_length=None, win_length=None, center=True):
     y, ptr = float_ptr(y)
     hop, win = _defaults(n_fft, hop_length, win_length)
     inter = bridge_call("mm_stft_complex", lib.mm_stft_complex, ptr, len(y), SR_UNUSED,
-                        stft_params(n_fft, hop, win, center))  # [n_freqs, n_frames, 2] float32
+                        stft_params(n_fft, hop, win, center),
+                        shape=frame_shape(n_fft // 2 + 1, len(y), n_fft, hop, center, 2))  # (re, im) pairs
     return np.ascontiguousarray(inter).view(np.complex64)[..., 0]
 
 
@@ -51,5 +53,6 @@ def istft(stft_matrix, hop_length=None, win_length=None, center=True, length=Non
     n_fft = (n_freqs - 1) * 2
     hop, win = _defaults(n_fft, hop_length, win_length)
     inter, ptr = float_ptr(np.ascontiguousarray(stft_matrix).view(np.float32))
+    length = length if length is not None else 0
     return bridge_call("mm_istft", lib.mm_istft, ptr, inter.size, n_freqs, n_frames, SR_UNUSED, hop, win,
-                       1 if center else 0, length if length is not None else 0)
+                       1 if center else 0, length, shape=sample_shape(n_frames, n_fft, hop, center, length))

@@ -23,13 +23,13 @@ struct Context {
   int magic = 0x4d4d4232;
 };
 std::mutex g_ctx_mu;
-std::unordered_map<const void *, bool> g_ctx;  // context -> its results may be pooled
+std::unordered_map<const void *, ResultPlace> g_ctx;
 
-mm_context new_context(bool pooled) {
+mm_context new_context(const ResultPlace &place) {
   Context *c = new (std::nothrow) Context();
   if (!c) return nullptr;
   std::lock_guard<std::mutex> lock(g_ctx_mu);
-  g_ctx[c] = pooled;
+  g_ctx[c] = place;
   return c;
 }
 
@@ -91,9 +91,10 @@ int run_batch(mm_context ctx, const Group &g_in, const float *const *signals, co
     return cuda_status(e);
   if ((e = enqueue_batch(g, L, t, b, s, nullptr, nullptr)) != cudaSuccess) return cuda_status(e);
   if (n == 1) {
-    if ((st = fetch_result(b.out, out_bytes, context_pooled(ctx), ws, &outs[0])) != MM_OK) return st;
+    const ResultPlace place = result_place(ctx);
+    if ((st = fetch_result(b.out, out_bytes, place, ws, &outs[0])) != MM_OK) return st;
     if ((st = take_error_word(g, t)) != MM_OK) {
-      result_free(outs[0]);
+      if (outs[0] != place.dst) result_free(outs[0]);
       outs[0] = nullptr;
     }
     return st;
@@ -139,17 +140,22 @@ bool supported_size(const Group &g) { return g.log2n <= 15; }
 
 }  // namespace
 
-bool mm::context_pooled(const void *ctx) {
+mm::ResultPlace mm::result_place(const void *ctx) {
   std::lock_guard<std::mutex> lock(g_ctx_mu);
   auto it = g_ctx.find(ctx);
-  return it != g_ctx.end() && it->second;
+  return it != g_ctx.end() ? it->second : ResultPlace{};
 }
 
 extern "C" {
 
-mm_context mm_init(void) { return new_context(false); }
+mm_context mm_init(void) { return new_context({}); }
 
-mm_context mm_init_pooled(void) { return new_context(true); }
+mm_context mm_init_pooled(void) { return new_context({true, nullptr, 0}); }
+
+mm_context mm_init_into(float *dst, int64_t count) {
+  if (!dst || count <= 0 || (uint64_t)count > SIZE_MAX / sizeof(float)) return nullptr;
+  return new_context({false, dst, sizeof(float) * (size_t)count});
+}
 
 void mm_destroy(mm_context ctx) {
   if (!ctx) return;
@@ -259,7 +265,7 @@ static int32_t db_common(mm_context ctx, const float *data, int64_t count, float
   if ((e = launch_db(d_x, d_y, count, mult, amin, ref, false, top_db, ws->dev + 2 * seg, s)) != cudaSuccess)
     return cuda_status(e);
   float *res = nullptr;
-  if ((st = fetch_result(d_y, bytes, context_pooled(ctx), ws, &res)) != MM_OK) return st;
+  if ((st = fetch_result(d_y, bytes, result_place(ctx), ws, &res)) != MM_OK) return st;
   fill_buffer(out, res, count, 0);
   out->ndim = 1;
   out->shape[1] = 0;
@@ -387,7 +393,7 @@ static int32_t run_matrix(mm_context ctx, const float *data, size_t in_count, si
   if (e == cudaSuccess) e = launch(d_in, d_out, s);
   if (e != cudaSuccess) return cuda_status(e);
   float *res = nullptr;
-  if ((st = fetch_result(d_out, out_b, context_pooled(ctx), ws, &res)) != MM_OK) return st;
+  if ((st = fetch_result(d_out, out_b, result_place(ctx), ws, &res)) != MM_OK) return st;
   fill_buffer(out, res, rows, cols);
   return MM_OK;
 }

@@ -196,7 +196,7 @@ int32_t mm_istft(mm_context ctx, const float *stft_data, int64_t stft_count, int
       cudaGetLastError();
       return cuda_status(e);
     }
-    if ((st = fetch_result(d_out, out_b, context_pooled(ctx), ws, &res)) != MM_OK) return st;
+    if ((st = fetch_result(d_out, out_b, result_place(ctx), ws, &res)) != MM_OK) return st;
   } else {
     res = (float *)calloc((size_t)out_len, sizeof(float));
     if (!res) return MM_ERR_ALLOC_FAILED;

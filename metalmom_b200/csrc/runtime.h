@@ -105,6 +105,7 @@ struct Workspace {
   size_t dev_bytes = 0;
   char *host = nullptr;
   size_t host_bytes = 0;
+  cudaEvent_t piece[4] = {};  // one per staging slot of fetch_result
 };
 // Returns the calling thread's workspace with at least the requested sizes.
 int thread_workspace(size_t dev_bytes, size_t host_bytes, Workspace **ws);
@@ -116,17 +117,24 @@ int thread_workspace(size_t dev_bytes, size_t host_bytes, Workspace **ws);
 // does not fit is malloc'd.
 float *result_alloc(size_t bytes, bool pooled, bool *pinned);
 void result_free(void *p);
+// Where a context's results go: page-locked blocks, the caller's own `dst`
+// when the size is exactly dst_bytes, else malloc.
+struct ResultPlace {
+  bool pooled = false;
+  float *dst = nullptr;
+  size_t dst_bytes = 0;
+};
+// That of `ctx` (malloc for anything unknown).
+ResultPlace result_place(const void *ctx);
 // Copy a device result to the host and wait for `s`: straight into a
 // page-locked block, else through the workspace's staging.
-int fetch_result(const float *d, size_t bytes, bool pooled, Workspace *ws, float **out);
+int fetch_result(const float *d, size_t bytes, const ResultPlace &place, Workspace *ws, float **out);
 // Enqueue the upload of host memory: large inputs straight from the caller's
 // buffer (the driver overlaps its own staging with the transfer), small ones
 // through the workspace's staging, at least upload_staging(bytes) long.
 constexpr size_t kDirectUpload = size_t(1) << 20;
 inline size_t upload_staging(size_t bytes) { return bytes < kDirectUpload ? bytes : 0; }
 cudaError_t upload(float *d, const float *h, size_t bytes, Workspace *ws);
-// Whether `ctx` came from mm_init_pooled (false for anything unknown).
-bool context_pooled(const void *ctx);
 
 // Fill an MMBuffer with a 2-D shape; data may be null when count is 0.
 void fill_buffer(MMBuffer *out, float *data, long long rows, long long cols);

@@ -155,7 +155,7 @@ int32_t run_columns(mm_context ctx, const float *S, int n_rows, long long T, int
     return cuda_status(e);
   }
   float *res = nullptr;
-  if ((st = fetch_result(d_out, out_b, context_pooled(ctx), ws, &res)) != MM_OK) return st;
+  if ((st = fetch_result(d_out, out_b, result_place(ctx), ws, &res)) != MM_OK) return st;
   fill_buffer(out, res, rows_out, T);
   return MM_OK;
 }

@@ -8,7 +8,7 @@ the GPU.
 
 import numpy as np
 
-from ._bridge import bridge_call as _call
+from ._bridge import bridge_call as _call, frame_shape
 from ._native import ffi, lib
 
 
@@ -42,7 +42,7 @@ def _mel_project(S, sr, n_fft, n_mels, fmin, fmax):
     c_fmax = float(fmax) if fmax is not None else 0.0
     ptr = ffi.cast("const float*", flat.ctypes.data)
     r = _call("mm_mel_project", lib.mm_mel_project, ptr, flat.size, flat.shape[0], flat.shape[1], sr, n_fft,
-              n_mels, float(fmin), c_fmax)
+              n_mels, float(fmin), c_fmax, shape=(n_mels, flat.shape[1]))
     return restore(r)
 
 
@@ -50,7 +50,8 @@ def _dct_ortho(S, n_mfcc):
     flat, restore = _columns(S, 0)
     n_out = len(range(flat.shape[0])[:n_mfcc])  # numpy slice semantics of [:n_mfcc]
     ptr = ffi.cast("const float*", flat.ctypes.data)
-    r = _call("mm_dct_ortho", lib.mm_dct_ortho, ptr, flat.size, flat.shape[0], flat.shape[1], n_out)
+    r = _call("mm_dct_ortho", lib.mm_dct_ortho, ptr, flat.size, flat.shape[0], flat.shape[1], n_out,
+              shape=(n_out, flat.shape[1]))
     return restore(r)
 
 
@@ -69,7 +70,8 @@ def melspectrogram(y=None, sr=22050, S=None, n_fft=2048, hop_length=None, win_le
     c_fmax = float(fmax) if fmax is not None else 0.0
     ptr = ffi.cast("const float*", y.ctypes.data)
     return _call("mm_mel_spectrogram", lib.mm_mel_spectrogram, ptr, len(y), sr, n_fft, hop, win,
-                 1 if center else 0, power, n_mels, fmin, c_fmax)
+                 1 if center else 0, power, n_mels, fmin, c_fmax,
+                 shape=frame_shape(n_mels, len(y), n_fft, hop, center))
 
 
 def mfcc(y=None, sr=22050, S=None, n_mfcc=20, n_fft=2048, hop_length=None, win_length=None,
@@ -87,7 +89,7 @@ def mfcc(y=None, sr=22050, S=None, n_mfcc=20, n_fft=2048, hop_length=None, win_l
     c_fmax = float(fmax) if fmax is not None else 0.0
     ptr = ffi.cast("const float*", y.ctypes.data)
     return _call("mm_mfcc", lib.mm_mfcc, ptr, len(y), sr, n_mfcc, n_fft, hop, win, n_mels, fmin,
-                 c_fmax, 1 if center else 0)
+                 c_fmax, 1 if center else 0, shape=frame_shape(min(n_mfcc, n_mels), len(y), n_fft, hop, center))
 
 
 def _db(name, fn, S, ref, amin, top_db):
@@ -98,7 +100,7 @@ def _db(name, fn, S, ref, amin, top_db):
     flat = S.ravel()
     c_top_db = float(top_db) if top_db is not None else 0.0
     ptr = ffi.cast("const float*", flat.ctypes.data)
-    return _call(name, fn, ptr, len(flat), ref, amin, c_top_db).reshape(shape)
+    return _call(name, fn, ptr, len(flat), ref, amin, c_top_db, shape=flat.shape).reshape(shape)
 
 
 def power_to_db(S, ref=1.0, amin=1e-10, top_db=80.0):
@@ -166,7 +168,7 @@ def delta(data, width=9, order=1, axis=-1, **kwargs):
     n_features, n_frames = data.shape
     flat = data.ravel()
     ptr = ffi.cast("const float*", flat.ctypes.data)
-    return _call("mm_delta", lib.mm_delta, ptr, len(flat), n_features, n_frames, width, order)
+    return _call("mm_delta", lib.mm_delta, ptr, len(flat), n_features, n_frames, width, order, shape=data.shape)
 
 
 def stack_memory(data, n_steps=2, delay=1, **kwargs):
@@ -179,4 +181,4 @@ def stack_memory(data, n_steps=2, delay=1, **kwargs):
     flat = data.ravel()
     ptr = ffi.cast("const float*", flat.ctypes.data)
     return _call("mm_stack_memory", lib.mm_stack_memory, ptr, len(flat), n_features, n_frames,
-                 n_steps, delay)
+                 n_steps, delay, shape=(n_features * n_steps, n_frames))

@@ -7,7 +7,7 @@ spectral flux is a kernel on the device.
 
 import numpy as np
 
-from .feature import _call
+from ._bridge import bridge_call as _call, frame_shape
 from ._native import ffi, lib
 
 
@@ -21,5 +21,6 @@ def onset_strength(y=None, sr=22050, S=None, n_fft=2048, hop_length=512, n_mels=
     c_fmax = float(fmax) if fmax is not None else 0.0
     ptr = ffi.cast("const float*", y.ctypes.data)
     res = _call("mm_onset_strength", lib.mm_onset_strength, ptr, len(y), sr, n_fft, hop_length, n_mels,
-                fmin, c_fmax, 1 if center else 0, 1 if aggregate else 0)
+                fmin, c_fmax, 1 if center else 0, 1 if aggregate else 0,
+                shape=frame_shape(1 if aggregate else n_mels, len(y), n_fft, hop_length, center))
     return res.ravel() if aggregate else res
