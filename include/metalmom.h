@@ -62,10 +62,8 @@ typedef void* mm_context;
 /* Replaces MetalMomBridge/Bridge.swift:22 (mm_init). */
 MM_API mm_context mm_init(void);
 
-/* Additive: as mm_init, but large results of calls on this context may lie in
- * page-locked blocks that the library keeps and reuses (64 MB at most; past
- * that they are malloc'd as usual), so that they arrive without a host copy.
- * Release them with mm_buffer_free and nothing else. */
+/* The same as mm_init, kept for callers of it: results used to lie in
+ * page-locked blocks that the library reused, and are malloc'd now. */
 MM_API mm_context mm_init_pooled(void);
 
 /* Additive: as mm_init, but a call on this context whose result has exactly

@@ -94,7 +94,7 @@ int run_batch(mm_context ctx, const Group &g_in, const float *const *signals, co
     const ResultPlace place = result_place(ctx);
     if ((st = fetch_result(b.out, out_bytes, place, ws, &outs[0])) != MM_OK) return st;
     if ((st = take_error_word(g, t)) != MM_OK) {
-      if (outs[0] != place.dst) result_free(outs[0]);
+      if (outs[0] != place.dst) free(outs[0]);
       outs[0] = nullptr;
     }
     return st;
@@ -150,11 +150,11 @@ extern "C" {
 
 mm_context mm_init(void) { return new_context({}); }
 
-mm_context mm_init_pooled(void) { return new_context({true, nullptr, 0}); }
+mm_context mm_init_pooled(void) { return new_context({}); }
 
 mm_context mm_init_into(float *dst, int64_t count) {
   if (!dst || count <= 0 || (uint64_t)count > SIZE_MAX / sizeof(float)) return nullptr;
-  return new_context({false, dst, sizeof(float) * (size_t)count});
+  return new_context({dst, sizeof(float) * (size_t)count});
 }
 
 void mm_destroy(mm_context ctx) {
@@ -168,7 +168,7 @@ void mm_destroy(mm_context ctx) {
 
 void mm_buffer_free(MMBuffer *buf) {
   if (!buf) return;
-  result_free(buf->data);
+  free(buf->data);
   buf->data = nullptr;
   buf->ndim = 0;
   buf->dtype = 0;

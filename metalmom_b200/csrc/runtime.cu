@@ -3,15 +3,12 @@
 
 #include <stdlib.h>
 #include <string.h>
-#include <sys/mman.h>
 
 #include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
-#include <unordered_map>
-#include <utility>
 #include <vector>
 
 namespace mm {
@@ -454,112 +451,8 @@ int thread_workspace(size_t dev_bytes, size_t host_bytes, Workspace **out) {
 // ---------------------------------------------------------------------------
 // host results
 // ---------------------------------------------------------------------------
-namespace {
-// Below kPoolMin the copies cost less than the bookkeeping; one block is at
-// most half of the cap, so that a result and the one before it both fit.
-constexpr size_t kPoolMin = size_t(256) << 10, kPoolCap = size_t(64) << 20;
 // Staging of a result on its way into pageable memory (see fetch_staged).
 constexpr size_t kFetchPiece = size_t(512) << 10, kFetchSlots = sizeof(Workspace::piece) / sizeof(cudaEvent_t);
-struct ResultPool {
-  std::mutex mu;
-  std::unordered_map<void *, size_t> live;  // handed out
-  std::multimap<size_t, void *> idle;
-  size_t total = 0;  // bytes of both
-  int refused = 0;   // requests since the last one that fitted
-};
-// never destroyed: results may be released while the process exits
-ResultPool &result_pool() {
-  static ResultPool *p = new ResultPool();
-  return *p;
-}
-// sizes are rounded up to a quarter of their power of two, so that calls on
-// clips of similar length share blocks
-size_t pool_class(size_t bytes) {
-  size_t step = kPoolMin / 4;
-  while (step * 8 < bytes) step *= 2;
-  return (bytes + step - 1) / step * step;
-}
-}  // namespace
-
-namespace {
-// Blocks are private anonymous memory, page-locked in place: after a fork the
-// child has copies of them as of any other memory (cudaHostAlloc's blocks were
-// shared, and a child's writes appeared in its parent's arrays).
-void *block_new(size_t bytes) {
-  void *p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_POPULATE, -1, 0);
-  if (p == MAP_FAILED) return nullptr;
-  if (cudaHostRegister(p, bytes, cudaHostRegisterPortable) == cudaSuccess) return p;
-  cudaGetLastError();
-  munmap(p, bytes);
-  return nullptr;
-}
-void block_delete(void *p, size_t bytes) {
-  // memory that could not be unlocked (a driver already shut down) stays mapped
-  if (cudaHostUnregister(p) == cudaSuccess) munmap(p, bytes);
-  else cudaGetLastError();
-}
-}  // namespace
-
-float *result_alloc(size_t bytes, bool pooled, bool *pinned) {
-  *pinned = false;
-  if (pooled && bytes >= kPoolMin && bytes <= kPoolCap / 2) {
-    ResultPool &rp = result_pool();
-    const size_t cls = pool_class(bytes);
-    std::vector<std::pair<size_t, void *>> drop;
-    bool fits = false;
-    {
-      std::lock_guard<std::mutex> lock(rp.mu);
-      auto it = rp.idle.find(cls);
-      if (it != rp.idle.end()) {
-        void *p = it->second;
-        rp.idle.erase(it);
-        rp.live[p] = cls;
-        rp.refused = 0;
-        *pinned = true;
-        return static_cast<float *>(p);
-      }
-      if (rp.total + cls > kPoolCap && ++rp.refused >= 16) {  // idle blocks of sizes no longer asked for
-        for (auto &b : rp.idle) {
-          rp.total -= b.first;
-          drop.push_back(b);
-        }
-        rp.idle.clear();
-        rp.refused = 0;
-      }
-      if (rp.total + cls <= kPoolCap) {
-        rp.total += cls;  // reserved while the block is made outside the lock
-        fits = true;
-      }
-    }
-    for (auto &b : drop) block_delete(b.second, b.first);
-    if (fits) {
-      void *p = block_new(cls);
-      std::lock_guard<std::mutex> lock(rp.mu);
-      if (p) {
-        rp.live[p] = cls;
-        *pinned = true;
-        return static_cast<float *>(p);
-      }
-      rp.total -= cls;
-    }
-  }
-  return static_cast<float *>(malloc(bytes));
-}
-
-void result_free(void *p) {
-  if (!p) return;
-  ResultPool &rp = result_pool();
-  {
-    std::lock_guard<std::mutex> lock(rp.mu);
-    auto it = rp.live.find(p);
-    if (it != rp.live.end()) {
-      rp.idle.emplace(it->second, p);
-      rp.live.erase(it);
-      return;
-    }
-  }
-  free(p);
-}
 
 // Through the staging in pieces, each copied on to `r` while the next ones cross
 // the bus.  Into memory that has been touched before, 5.3 MB / 2.6 MB / 0.66 MB
@@ -572,7 +465,7 @@ static cudaError_t fetch_staged(const float *d, size_t bytes, Workspace *ws, flo
   const char *src = reinterpret_cast<const char *>(d);
   char *dst = reinterpret_cast<char *>(r);
   const size_t pieces = (bytes + kPiece - 1) / kPiece;
-  if (pieces == 1) {
+  if (pieces <= 1) {
     cudaError_t e = cudaMemcpyAsync(ws->host, src, bytes, cudaMemcpyDeviceToHost, ws->stream);
     const cudaError_t e2 = cudaStreamSynchronize(ws->stream);
     if (e == cudaSuccess) e = e2;
@@ -597,27 +490,16 @@ static cudaError_t fetch_staged(const float *d, size_t bytes, Workspace *ws, flo
 }
 
 int fetch_result(const float *d, size_t bytes, const ResultPlace &place, Workspace *ws, float **out) {
+  Workspace *same = nullptr;  // waits for the stream if the staging has to grow
+  const int st = thread_workspace(0, std::min(bytes, kFetchPiece * kFetchSlots), &same);
+  if (st != MM_OK) return st;
   const bool given = place.dst && place.dst_bytes == bytes;
-  bool pinned = false;
-  float *r = given ? place.dst : result_alloc(bytes, place.pooled, &pinned);
+  float *r = given ? place.dst : static_cast<float *>(malloc(bytes));
   if (!r) return MM_ERR_ALLOC_FAILED;
-  cudaError_t e = cudaSuccess;
-  if (pinned) {
-    e = cudaMemcpyAsync(r, d, bytes, cudaMemcpyDeviceToHost, ws->stream);
-    const cudaError_t e2 = cudaStreamSynchronize(ws->stream);
-    if (e == cudaSuccess) e = e2;
-  } else {
-    Workspace *same = nullptr;  // waits for the stream if the staging has to grow
-    const int st = thread_workspace(0, std::min(bytes, kFetchPiece * kFetchSlots), &same);
-    if (st != MM_OK) {
-      if (!given) result_free(r);
-      return st;
-    }
-    e = fetch_staged(d, bytes, ws, r);
-  }
+  const cudaError_t e = fetch_staged(d, bytes, ws, r);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    if (!given) result_free(r);
+    if (!given) free(r);
     return cuda_status(e);
   }
   *out = r;

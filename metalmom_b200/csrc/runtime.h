@@ -110,24 +110,16 @@ struct Workspace {
 // Returns the calling thread's workspace with at least the requested sizes.
 int thread_workspace(size_t dev_bytes, size_t host_bytes, Workspace **ws);
 
-// Host results.  result_alloc returns malloc'd memory, or, where `pooled` and
-// the size make it worth while, a page-locked block of the library's pool
-// (*pinned), which the device writes directly; result_free gives either back
-// (thread-safe).  The pool holds at most 64 MB in use and idle together; what
-// does not fit is malloc'd.
-float *result_alloc(size_t bytes, bool pooled, bool *pinned);
-void result_free(void *p);
-// Where a context's results go: page-locked blocks, the caller's own `dst`
-// when the size is exactly dst_bytes, else malloc.
+// Where a context's results go: the caller's own `dst` when the size is exactly
+// dst_bytes, else malloc.
 struct ResultPlace {
-  bool pooled = false;
   float *dst = nullptr;
   size_t dst_bytes = 0;
 };
 // That of `ctx` (malloc for anything unknown).
 ResultPlace result_place(const void *ctx);
-// Copy a device result to the host and wait for `s`: straight into a
-// page-locked block, else through the workspace's staging.
+// Copy a device result to its place through the workspace's staging and wait
+// for the stream.
 int fetch_result(const float *d, size_t bytes, const ResultPlace &place, Workspace *ws, float **out);
 // Enqueue the upload of host memory: large inputs straight from the caller's
 // buffer (the driver overlaps its own staging with the transfer), small ones
