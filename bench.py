@@ -913,7 +913,7 @@ def kernel_case(args):
     b.record(stream)
     torch.cuda.synchronize()
     out = {"kernel_case": {"n_fft": n_fft, "hop_length": n_fft // 4, "clips": args.clips,
-                           "variant": M.tune_get(n_fft), "ms_per_step": a.elapsed_time(b) / max(args.steps, 1)}}
+                           "variant": M.tune_variant(n_fft), "ms_per_step": a.elapsed_time(b) / max(args.steps, 1)}}
     plan.close()
     return out
 

@@ -288,9 +288,10 @@ MM_API int32_t mm_plan_execute_host(mm_plan plan, const float* const* signals, f
  * clips of clip_samples samples (reps launches each), writes each variant's
  * milliseconds to variant_ms[variant] (6 entries; 0 for variants not timed),
  * keeps the fastest and returns it in *best_variant.  Plans and calls made
- * afterwards use the tuned variant.  A size that neither mm_autotune nor
- * mm_tune_set has set runs variant 3 wherever it exists and variant 0
- * elsewhere; mm_tune_get still reports 0 there below n_fft 2048. */
+ * afterwards use the tuned variant.  mm_tune_get reports the variant that MFCC
+ * calls at n_fft run: 3 for n_fft 256..4096 and 0 elsewhere until mm_autotune
+ * or mm_tune_set has set another, so that setting back what was read restores
+ * the library's own choice. */
 MM_API int32_t mm_autotune(mm_context ctx, const MMFrontEndParams* params, int64_t clip_samples,
                            int32_t n_clips, int32_t reps, float* variant_ms, int32_t* best_variant);
 MM_API int32_t mm_tune_set(int32_t n_fft, int32_t variant);

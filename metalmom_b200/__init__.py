@@ -21,7 +21,7 @@ _API = {
     "stack_memory": "feature",
     "onset_strength": "onset",
     "mfcc_batch": "batch", "Plan": "batch", "frontend_params": "batch", "autotune": "batch",
-    "tune_get": "batch", "tune_set": "batch",
+    "tune_get": "batch", "tune_set": "batch", "tune_variant": "batch",
     "Server": "serve",
 }
 

@@ -33,6 +33,16 @@ def frontend_params(sr=22050, n_fft=2048, hop_length=None, win_length=None, cent
     return p
 
 
+_tuned = set()  # the n_fft that tune_set or autotune has set
+
+
+class _Untuned(int):
+    """What ``tune_get`` returns for an n_fft that nothing has set where the
+    library's own choice has another number: ``variant``."""
+
+    variant = 0
+
+
 def autotune(clip_samples=661500, n_clips=32, reps=10, **params):
     """Time every launch variant of the frame kernel for these parameters on
     synthetic clips, keep the fastest for this n_fft (process-wide) and return
@@ -47,17 +57,43 @@ def autotune(clip_samples=661500, n_clips=32, reps=10, **params):
             raise RuntimeError(f"mm_autotune failed with status {st}")
     finally:
         lib.mm_destroy(ctx)
+    _tuned.add(p.n_fft)
     return {"best": int(best[0]), "ms": {i: float(ms[i]) for i in range(6) if ms[i] > 0}}
 
 
 def tune_set(n_fft, variant):
-    st = lib.mm_tune_set(n_fft, variant)
+    """Fix the frame kernel's launch variant for n_fft (process-wide), or set
+    back what ``tune_get`` returned."""
+    back = isinstance(variant, _Untuned) and 256 <= n_fft <= 1024
+    st = lib.mm_tune_set(n_fft, variant.variant if back else variant)
     if st != 0:
         raise RuntimeError(f"mm_tune_set failed with status {st}")
+    if back:
+        _tuned.discard(n_fft)
+    else:
+        _tuned.add(n_fft)
 
 
 def tune_get(n_fft):
-    return int(lib.mm_tune_get(n_fft))
+    """The setting of n_fft, for ``tune_set`` to restore: the variant that
+    ``tune_set`` or ``autotune`` set.  For an n_fft that neither has set it is
+    the number this function has always given there (3 for 2048 and 4096, else
+    0), for 256..1024 as a marked 0, since MFCC calls run variant 3 there:
+    ``tune_variant`` tells what runs."""
+    v = int(lib.mm_tune_get(n_fft))
+    if v == 3 and 256 <= n_fft <= 1024 and n_fft not in _tuned:
+        untuned = _Untuned(0)
+        untuned.variant = v
+        return untuned
+    return v
+
+
+def tune_variant(n_fft):
+    """The launch variant that MFCC calls and plans made now run at n_fft."""
+    v = int(lib.mm_tune_get(n_fft))
+    if v < 0:
+        raise RuntimeError(f"mm_tune_get failed with status {v}")
+    return v
 
 
 def mfcc_batch(clips, **params):

@@ -36,27 +36,23 @@ int gpu_available() {
 }
 
 namespace {
-// What mm_tune_set or mm_autotune last stored per log2(n_fft), as mm_tune_get
-// reports it, and whether either has run for that size.
-std::atomic<int> g_tuned[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, kWarpVariant, kWarpVariant, 0, 0, 0};
-std::atomic<bool> g_tuned_set[16];
+// Launch variant per log2(n_fft) until mm_tune_set or mm_autotune stores
+// another: variant 3 for n_fft 256..4096, 0 elsewhere; a mode without variant
+// 3 falls back to 0.  Whole step against variant 0 on 64 clips of 30 s (hop
+// n_fft/4): n_fft 256 323 / 520 us, 512 253 / 410, 1024 225 / 441, 2048 218 /
+// 428, 4096 289 / 449; on one clip of 1 to 30 s between equal and 1.5x faster
+// (n_fft 256 and 512 with few frames: within one 2 us step either way).
+std::atomic<int> g_tuned[16] = {0, 0, 0, 0, 0, 0, 0, 0, kWarpVariant, kWarpVariant, kWarpVariant, kWarpVariant,
+                                kWarpVariant, 0, 0, 0};
 }
 
 int tuned_variant(int log2n) { return (log2n >= 0 && log2n < 16) ? g_tuned[log2n].load() : 0; }
 void set_tuned_variant(int log2n, int v) {
-  if (log2n < 0 || log2n >= 16) return;
-  g_tuned[log2n].store(v);
-  g_tuned_set[log2n].store(true);
+  if (log2n >= 0 && log2n < 16) g_tuned[log2n].store(v);
 }
 int group_variant(const Group &g) {
   if (g.dft_form != DFT_FFT_F32) return kDftVariant;
   const int nv = frame_variants(g.log2n, g.mode, g.power == 2.0f);
-  // Untuned: variant 3 wherever it exists (MFCC path, n_fft 256..4096).  Whole
-  // step against variant 0 on 64 clips of 30 s (hop n_fft/4): n_fft 256 323 /
-  // 520 us, 512 253 / 410, 1024 225 / 441, 2048 218 / 428, 4096 289 / 449; on
-  // one clip of 1 to 30 s between equal and 1.5x faster (n_fft 256 and 512 with
-  // few frames: within one 2 us step either way).
-  if (g.log2n < 16 && !g_tuned_set[g.log2n].load()) return nv > kWarpVariant ? kWarpVariant : 0;
   const int v = tuned_variant(g.log2n);
   if (v == kTcVariant)  // the tensor-core kernel: n_fft 2048 on the MFCC path only
     return (g.log2n == 11 && g.mode == MODE_MELDB && g.power == 2.0f) ? kTcVariant : (nv > kWarpVariant ? kWarpVariant : 0);
