@@ -9,11 +9,13 @@ import pytest
 import metalmom_b200 as M
 from goldens import golden, signal_440
 from metalmom_b200 import synth
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
 SR = 22050
 SIZES = [256, 512, 1024, 2048, 4096]
+MFCC_TOL = 1e-4  # of max |c|, as every MFCC test
 
 
 @pytest.fixture
@@ -80,3 +82,22 @@ def test_the_reference_golden_at_1024(variant):
     variant(1024, 3)
     got = M.mfcc(y=signal_440(), sr=SR, n_mfcc=13, n_fft=1024, n_mels=40)
     np.testing.assert_allclose(got, golden("mfcc_440hz_13_1024"), rtol=1e-4, atol=1e-4)
+
+@pytest.mark.parametrize("center", [True, False])
+@pytest.mark.parametrize("n_fft,hop,n_mels", [
+    (256, 64, 40), (256, 80, 40), (256, 85, 26), (256, 128, 26), (512, 128, 40), (512, 160, 80), (512, 256, 80),
+    (1024, 256, 64), (1024, 320, 64), (1024, 441, 64), (1024, 512, 64), (2048, 512, 128), (2048, 441, 128),
+    (2048, 1024, 40), (4096, 1024, 128), (4096, 441, 64), (4096, 2048, 40),
+])
+def test_reflected_edges_vs_oracle(n_fft, hop, n_mels, center, variant):
+    """Both edges of clips from just over the padding (one reflection) to many
+    frames, odd lengths among them."""
+    variant(n_fft, 3)
+    lens = [n_fft // 2 + 1, n_fft, n_fft + hop, 2 * n_fft + 3, n_fft + 7 * hop + 1]
+    clips = [synth.music_clip(n, SR, seed=n + hop) for n in lens]
+    params = dict(sr=SR, n_fft=n_fft, hop_length=hop, n_mels=n_mels, center=center, pad_mode="reflect")
+    for y, got in zip(clips, M.mfcc_batch(clips, **params)):
+        exp = O.mfcc(y, SR, min(20, n_mels), n_fft, hop, n_fft, n_mels, center=center, pad_mode=O.PAD_REFLECT)
+        assert got.shape == exp.shape, len(y)
+        if exp.size:
+            assert O.mfcc_rel_error(got, exp) < MFCC_TOL, (len(y), O.mfcc_rel_error(got, exp))
