@@ -197,29 +197,6 @@ __device__ __forceinline__ void dft16(cpx2 *v) {
   for (int i = 0; i < 16; i++) v[i] = o[i];
 }
 
-// The same in eight steps of one 4-point DFT each (the reordering comes with
-// the last), for code that interleaves them with other work.
-template <int ST>
-__device__ __forceinline__ void dft16_step(cpx2 *v) {
-  if constexpr (ST < 4) {
-    dft4(v[ST], v[ST + 4], v[ST + 8], v[ST + 12]);
-  } else if constexpr (ST == 4) {
-    dft4(v[0], v[1], v[2], v[3]);
-  } else {
-    constexpr int k = ST - 4;
-    dft4_tw<k, 16>(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-  }
-  if constexpr (ST == 7) {
-    cpx2 o[16];
-#pragma unroll
-    for (int k1 = 0; k1 < 4; k1++)
-#pragma unroll
-      for (int k2 = 0; k2 < 4; k2++) o[k1 + 4 * k2] = v[4 * k1 + k2];
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = o[i];
-  }
-}
-
 // In-place 32-point DFT, natural order: radix-2 over two 16-point DFTs (380
 // operations, 444 with separate twiddle products).
 __device__ __forceinline__ void dft32(cpx2 *v) {

@@ -19,6 +19,16 @@
 
 namespace mm {
 
+// Samples (x[i], x[i+1]) for i = first + stride r, r < 32, with the padding
+// rule of sample_at; used only for frames that overlap the clip's edges.
+static __device__ __noinline__ void gather_edge(cpx *out, const float *sig, long long first, long long length,
+                                         int pad_mode, int stride) {
+  for (int r = 0; r < 32; r++) {
+    const long long n0 = first + (long long)stride * r;
+    out[r] = {sample_at(sig, n0, length, pad_mode), sample_at(sig, n0 + 1, length, pad_mode)};
+  }
+}
+
 // Position of bin k in the padded power spectrum: PS floats per 32 bins,
 // k + (PS - 32) min(k / 32, TPF - 1).
 template <int TPF, int PS = 33>

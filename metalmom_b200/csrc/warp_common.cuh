@@ -1,6 +1,6 @@
-// Device helpers shared by the warp-per-frame kernels: compile-time roots of
-// unity, the quarter-table root lookup, the gather of frames that reach into
-// the padding, stage-2 column assignment.
+// Device helpers shared by the frame-pair and tensor-core frame kernels:
+// compile-time roots of unity, the quarter-table root lookup, stage-2 column
+// assignment.
 #pragma once
 #include <math.h>
 
@@ -103,17 +103,7 @@ __device__ __forceinline__ cpx root_q(const float2 *q, int s, int N) {
   }
 }
 
-// Samples (x[i], x[i+1]) for i = first + stride r, r < 32, with the padding
-// rule of sample_at; used only for frames that overlap the clip's edges.
-static __device__ __noinline__ void gather_edge(cpx *out, const float *sig, long long first, long long length,
-                                         int pad_mode, int stride) {
-  for (int r = 0; r < 32; r++) {
-    const long long n0 = first + (long long)stride * r;
-    out[r] = {sample_at(sig, n0, length, pad_mode), sample_at(sig, n0 + 1, length, pad_mode)};
-  }
-}
-
-// stage-2 column of slot c for lane l (see the header comment)
+// Stage-2 column of slot c for lane l: columns k1 and 32 - k1 sit in one lane.
 template <int TPF, int C, int c>
 __device__ __forceinline__ int stage2_col(int l) {
   if constexpr (C == 1) {
