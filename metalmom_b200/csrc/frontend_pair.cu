@@ -969,17 +969,19 @@ static cudaError_t launch_pair4096_d(const FrontArgs &a, int grid_limit, cudaStr
   return launch_units(frame_pair4096_kernel<D>, a, S::UT, S::NP, 64 * S::NP, smem_of, grid_limit, s, launched);
 }
 
-// Shared gathers exist for the usual hops, each against D = 0 on 64 clips of
-// 30 s (whole step): n_fft/2 at n_fft 256 195 -> 181 us, 512 147 -> 139, 1024
-// 134 -> 135 (one clip: 17.5 -> 16.6), 2048 125 -> 121; 10 ms of 32 ms at n_fft
-// 256 304 -> 274, 512 225 -> 209, 1024 198 -> 197; 512 utterances of 10 s at
-// n_fft 512 420 -> 394.
+// Shared gathers exist for the usual hops where they win, against D = 0 on 256
+// clips of 15 s (whole step, us): n_fft/4 at n_fft 256 640 / 707, 512 483 / 515,
+// 1024 451 / 461, 2048 413 / 427, 4096 513 / 535; n_fft/2 at 256 348 / 376, 512
+// 265 / 278, 2048 227 / 234; 10 ms of 32 ms at 256 526 / 581, 512 402 / 426.  At n_fft
+// 1024 neither of the last two does: 256 clips of 30 s 481 / 478 (n_fft/2) and
+// 743 / 736 (10 ms of 32 ms), one clip 16.5 us in every form.
 template <int LOG2N>
 static cudaError_t launch_pair(const FrontArgs &a, int grid_limit, cudaStream_t s, int *launched) {
   constexpr int step = 2 * PShape<LOG2N>::TPF;  // samples per register step, n_fft / 32
   if (a.even_starts && a.hop == 8 * step) return launch_pair_d<LOG2N, 8>(a, grid_limit, s, launched);    // n_fft / 4
-  if (a.even_starts && a.hop == 16 * step) return launch_pair_d<LOG2N, 16>(a, grid_limit, s, launched);  // n_fft / 2
-  if constexpr (LOG2N <= 10)  // 10 ms of a 32 ms frame: speech at 8, 16 and 32 kHz
+  if constexpr (LOG2N != 10)  // n_fft / 2
+    if (a.even_starts && a.hop == 16 * step) return launch_pair_d<LOG2N, 16>(a, grid_limit, s, launched);
+  if constexpr (LOG2N <= 9)  // 10 ms of a 32 ms frame: speech at 8 and 16 kHz
     if (a.even_starts && a.hop == 10 * step) return launch_pair_d<LOG2N, 10>(a, grid_limit, s, launched);
   return launch_pair_d<LOG2N, 0>(a, grid_limit, s, launched);
 }
