@@ -500,6 +500,23 @@ def uneven_shard(work, rank, world):
     return sorted(shards[rank])
 
 
+def frame_kernel_name(variant):
+    """The frame kernel that a launch variant is on the headline workload."""
+    return {3: "frame_pair_kernel<11>", 5: "frame_tc_kernel"}.get(variant, f"frontend_kernel<11,V{variant},MELDB>")
+
+
+def recorded_traffic(kname):
+    """DRAM bytes per launch on the headline workload, as profiled; None where
+    that kernel has no record."""
+    path = os.path.join(ROOT, "profiles", kname.split("<")[0] + "_256clips_traffic.txt")
+    if not os.path.exists(path):
+        return None
+    for line in open(path):
+        if line.startswith("bytes_per_launch:"):
+            return float(line.split(":")[1])
+    return None
+
+
 def uneven_leg(stream, rank=0, world=1, dist=None, steps=20, n_clips=1024, seed=2024, variant=None):
     """The uneven batch: 1024 clips, lengths uniform in 1-120 s, each clip
     with its own group (sr 22050/44100, n_fft 1024/2048/4096 with hop n_fft/4,
@@ -778,15 +795,8 @@ def run_ours(args, rank, world, local_rank):
         achieved = alg_bytes / (frame_ms / 1e3) / 1e9
         pipe_bytes = 4.0 * sum(lengths) + 4.0 * N_MFCC * T_total
         flops_fft = 2.5 * N_FFT * np.log2(N_FFT) * T_total
-        traffic = None
-        warp = tune["best"] == 3
-        kname = {3: "frame_pair_kernel<11>", 5: "frame_tc_kernel"}.get(
-            tune["best"], f"frontend_kernel<11,V{tune['best']},MELDB>")
-        tp = os.path.join(ROOT, "profiles", kname.split("<")[0] + "_256clips_traffic.txt")
-        if os.path.exists(tp) and n_clips == N_CLIPS:
-            for line in open(tp):
-                if line.startswith("bytes_per_launch:"):
-                    traffic = float(line.split(":")[1])
+        kname = frame_kernel_name(tune["best"])
+        traffic = recorded_traffic(kname) if n_clips == N_CLIPS else None
         result = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K,
             "warmup": W, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
