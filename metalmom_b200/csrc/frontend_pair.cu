@@ -37,9 +37,9 @@
 // the issue slots: 2 075 -> 1 200 warp instructions and ~610 -> 480
 // shared-memory wavefronts a frame.  The price is the register file: 128
 // registers of data a lane leave 8 warps an SM, and with two warps a scheduler
-// the kernel now waits on its own latencies (issue 44 %, shared-memory pipe
-// 67 %).  256 clips of 30 s at n_fft 2048, hop 512, 128 bands: 0.90 -> 0.77 ms
-// (whole step 0.954 -> 0.833); 512 clips of 10 s at n_fft 512, hop 160, 80
+// the kernel now waits on its own latencies (issue 45 %, L1 / shared-memory
+// pipe 74 %).  256 clips of 30 s at n_fft 2048, hop 512, 128 bands: 0.90 -> 0.76
+// ms (whole step 0.954 -> 0.81); 512 clips of 10 s at n_fft 512, hop 160, 80
 // bands, whole step: 0.62 (CTA-tile kernel) -> 0.39.  64 clips of 30 s at 44.1 kHz,
 // n_fft 4096, hop 1024: 0.571 -> 0.511 (one frame per warp pair, 16 warps, before).
 // Measured and left out (128 clips, whole step, against 0.426 ms): 12 warps of

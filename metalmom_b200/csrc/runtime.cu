@@ -455,7 +455,9 @@ constexpr size_t kFetchPiece = size_t(512) << 10, kFetchSlots = sizeof(Workspace
 // take 342 / 179 / 46 us; the whole result staged first 398 / 205 / 47, a copy by
 // the driver into the pageable memory itself 287 / 158 / 58 but, where the
 // pages are new, 2 409 / 1 200 / 321 against 1 441 / 733 / 187.  Pieces of 256 KB
-// 365 / 189 / 45, of 1 MB 334 / 179 / 47.
+// 365 / 189 / 45, of 1 MB 334 / 179 / 47.  Measured and left out: non-temporal
+// stores (311 / 165 / 56), three threads sharing the pieces (209 / 121 / 50, but
+// 90th percentiles of 670 / 430 / 72 against 354 / 186 / 48).
 static cudaError_t fetch_staged(const float *d, size_t bytes, Workspace *ws, float *r) {
   constexpr size_t kPiece = kFetchPiece, kSlots = kFetchSlots;
   const char *src = reinterpret_cast<const char *>(d);
